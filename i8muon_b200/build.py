@@ -9,18 +9,18 @@ from __future__ import annotations
 import os
 import shutil
 import subprocess
+import tempfile
+from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
 CSRC = Path(__file__).resolve().parent / "csrc"
 LIBRARY = CSRC / "libi8muon_b200.so"
-SOURCES = ("ns_api.cu",)
-HEADERS = ("ptx_sm100.cuh", "gemm_core.cuh", "gemm_bq_persistent.cuh", "gemm_wholek_persistent.cuh", "epi_float.cuh", "epi_int8.cuh", "epi_bq.cuh",
-           "passes.cuh")
+SOURCES = ("ns_api.cu", "api_float.cu", "api_int8.cu", "api_bq.cu", "api_passes.cu")
 NVCC_FLAGS = (
     "-std=c++17", "-O3", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",
     # FP32 expressions are evaluated exactly as written; fused multiply-adds
     # appear only where the code asks for them.
-    "--fmad=false", "-Xcompiler", "-fPIC", "-shared",
+    "--fmad=false", "-Xcompiler", "-fPIC",
 )
 
 
@@ -36,23 +36,32 @@ def needs_build() -> bool:
         return True
     built = LIBRARY.stat().st_mtime
     header = Path(__file__).resolve().parents[1] / "include" / "i8muon_b200.h"
-    deps = [CSRC / name for name in SOURCES + HEADERS] + [header]
+    deps = [*CSRC.glob("*.cu"), *CSRC.glob("*.cuh"), header]
     return any(dep.stat().st_mtime > built for dep in deps)
 
 
-def build(force: bool = False, verbose: bool = False) -> Path:
-    """Compile ``csrc/*.cu`` into ``csrc/libi8muon_b200.so`` for sm_100a."""
-    if not force and not needs_build():
-        return LIBRARY
-    command = [_nvcc(), *NVCC_FLAGS, "-o", str(LIBRARY), *[str(CSRC / s) for s in SOURCES]]
-    if verbose or os.environ.get("I8MUON_BUILD_VERBOSE", "0") not in ("", "0"):
-        command.insert(1, "-Xptxas=-v")
-        print(" ".join(command))
+def _compile(source: str, output: Path, verbose: bool) -> str:
+    command = [_nvcc(), *NVCC_FLAGS, *(["-Xptxas=-v"] if verbose else []), "-c", "-o", str(output), str(CSRC / source)]
     result = subprocess.run(command, capture_output=True, text=True)
     if result.returncode != 0:
-        raise RuntimeError(f"nvcc failed:\n{result.stdout}\n{result.stderr}")
+        raise RuntimeError(f"nvcc failed on {source}:\n{result.stdout}\n{result.stderr}")
+    return " ".join(command) + "\n" + result.stderr
+
+
+def build(force: bool = False, verbose: bool = False) -> Path:
+    """Compile ``csrc/*.cu`` (one nvcc process per file, in parallel) into ``csrc/libi8muon_b200.so`` for sm_100a."""
+    if not force and not needs_build():
+        return LIBRARY
+    verbose = verbose or os.environ.get("I8MUON_BUILD_VERBOSE", "0") not in ("", "0")
+    with tempfile.TemporaryDirectory() as work, ThreadPoolExecutor(len(SOURCES)) as pool:
+        objects = [Path(work) / (source + ".o") for source in SOURCES]
+        logs = list(pool.map(_compile, SOURCES, objects, [verbose] * len(SOURCES)))
+        link = [_nvcc(), *NVCC_FLAGS, "-shared", "-o", str(LIBRARY), *map(str, objects)]
+        result = subprocess.run(link, capture_output=True, text=True)
+    if result.returncode != 0:
+        raise RuntimeError(f"linking failed:\n{result.stdout}\n{result.stderr}")
     if verbose:
-        print(result.stderr)
+        print("\n".join(logs))
     return LIBRARY
 
 

@@ -79,6 +79,7 @@ bq_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_wait();
   const uint32_t tmem_base = ctrl->tmem_base;
   volatile uint32_t* abort_flag = &ctrl->abort;
   const uint32_t smem_base = smem_u32(smem);

@@ -1,0 +1,133 @@
+// Launch templates of the GEMM kernels: one place that fills the geometry, encodes the operand maps and picks the
+// kernel for an epilogue.
+#pragma once
+#include "host.cuh"
+#include "gemm_bq_persistent.cuh"
+#include "gemm_bq_split.cuh"
+#include "gemm_wholek_persistent.cuh"
+#include "gemm_wholek_wide.cuh"
+
+namespace i8m {
+
+// Row blocks per group of the wide-unit order: as many as keep the group's left row blocks
+// (128 rows x k bytes each) within 32 MB of L2; even, 8 to 64.
+inline int wide_group(long long k_bytes) {
+  const long long fit = (32LL << 20) / std::max<long long>(1, 128 * k_bytes);
+  return int(std::min<long long>(64, std::max<long long>(8, fit))) & ~1;
+}
+
+template <class Epi>
+int launch_gemm(const void* a, const void* a_lo, const void* bt, const void* bt_lo, int batch,
+                int m, int n, int k, int lm, int ln, int sym, unsigned* status,
+                const typename Epi::Args& args, cudaStream_t stream, const char* name) {
+  if (batch < 1 || m < 1 || n < 1 || k < 1) return fail(I8M_E_ARGUMENT, "%s: empty problem", name);
+  if (!a || !bt || !status) return fail(I8M_E_ARGUMENT, "%s: null operand or status pointer", name);
+  if (sym && m != n) return fail(I8M_E_ARGUMENT, "%s: symmetric product needs m == n", name);
+  constexpr int ES = int(sizeof(typename Epi::Elem));
+  constexpr int STAGE_BYTES = 2 * Epi::PARTS * TILE_BYTES;
+  constexpr size_t SMEM = size_t(Epi::STAGES) * STAGE_BYTES + sizeof(Ctrl) + 1024;
+  GemmGeom g;
+  g.batch = batch; g.m = m; g.n = n; g.k = k; g.lm = lm; g.ln = ln;
+  g.tiles_m = cdiv(m, TILE); g.tiles_n = cdiv(n, TILE);
+  g.sym = sym;
+  g.tiles_per_batch = sym ? g.tiles_m * (g.tiles_m + 1) / 2 : g.tiles_m * g.tiles_n;
+  g.num_kb = cdiv((long long)k * ES, 128);
+  g.debug_simt = g_debug_simt | (g_starve_producers ? 0x100 : 0);
+  g.group = wide_group((long long)k * ES);
+  g.a_raw = a; g.b_raw = bt; g.status = status;
+  long long blocks = (long long)g.tiles_per_batch * batch;
+  if (blocks > 0x7fffffffLL) return fail(I8M_E_LIMIT, "%s: too many tiles", name);
+  CUtensorMap ma, mb, ma2, mb2;
+  if (int rc = make_operand_map(&ma, a, ES, k, m, batch)) return rc;
+  if (int rc = make_operand_map(&mb, bt, ES, k, n, batch)) return rc;
+  if (Epi::PARTS == 2) {
+    if (!a_lo || !bt_lo) return fail(I8M_E_ARGUMENT, "%s: missing low planes", name);
+    if (int rc = make_operand_map(&ma2, a_lo, ES, k, m, batch)) return rc;
+    if (int rc = make_operand_map(&mb2, bt_lo, ES, k, n, batch)) return rc;
+  } else {
+    ma2 = ma; mb2 = mb;
+  }
+  // products that accumulate their whole K extent in tensor memory: persistent kernel
+  if constexpr (!Epi::BLOCKQ && Epi::PARTS == 1 && Epi::PROMOTE_KB == 0) {
+    if (!g_debug_simt && g_wholek_variant == 0) {
+      constexpr size_t WSMEM = wholek_wide_smem_bytes<Epi>();
+      auto wk = wholek_wide_kernel<Epi>;
+      static SmemAllowed allowed;
+      if (int rc = allow_smem(allowed, wk, WSMEM)) return rc;
+      const long long units = (long long)wide_units_per_batch(g.tiles_m, g.tiles_n, sym) * batch;
+      launch(wk, unsigned(std::min<long long>(units, sm_count())), WKW_THREADS, WSMEM, stream, ma, mb, g, args);
+      LAUNCH_CHECK(name);
+      return 0;
+    }
+    if (!g_debug_simt && g_wholek_variant == 1) {
+      constexpr size_t PSMEM = size_t(WKP_STAGES) * 2 * TILE_BYTES + sizeof(Ctrl) + 1024;
+      auto pk = wholek_persistent_kernel<Epi>;
+      static SmemAllowed allowed;
+      if (int rc = allow_smem(allowed, pk, PSMEM)) return rc;
+      const unsigned grid = unsigned(std::min<long long>(blocks, sm_count()));
+      launch(pk, grid, WKP_THREADS, PSMEM, stream, ma, mb, g, args);
+      LAUNCH_CHECK(name);
+      return 0;
+    }
+  }
+  auto kernel = ns_gemm_kernel<Epi, true>;
+  if constexpr (!Epi::BLOCKQ) {
+    if (!g_debug_simt) kernel = ns_gemm_kernel<Epi, false>;
+  }
+  static SmemAllowed allowed[2];
+  if (int rc = allow_smem(allowed[g_debug_simt != 0], kernel, SMEM)) return rc;
+  launch(kernel, dim3(unsigned(blocks)), WarpLayout<Epi>::THREADS, SMEM, stream, ma, mb, ma2, mb2, g, args);
+  LAUNCH_CHECK(name);
+  return 0;
+}
+
+// Block-quantised GEMMs: persistent kernel, one CTA per SM (the debug core keeps the
+// one-tile-per-CTA skeleton).
+template <class Epi>
+int launch_bq(const void* a, const void* bt, int batch, int m, int n, int k, int lm, int ln, int sym,
+              unsigned* status, const typename Epi::Args& args, cudaStream_t stream, const char* name) {
+  if (g_debug_simt)
+    return launch_gemm<Epi>(a, nullptr, bt, nullptr, batch, m, n, k, lm, ln, sym, status, args, stream, name);
+  if (batch < 1 || m < 1 || n < 1 || k < 1) return fail(I8M_E_ARGUMENT, "%s: empty problem", name);
+  if (!a || !bt || !status) return fail(I8M_E_ARGUMENT, "%s: null operand or status pointer", name);
+  if (sym && m != n) return fail(I8M_E_ARGUMENT, "%s: symmetric product needs m == n", name);
+  GemmGeom g;
+  g.batch = batch; g.m = m; g.n = n; g.k = k; g.lm = lm; g.ln = ln;
+  g.tiles_m = cdiv(m, TILE); g.tiles_n = cdiv(n, TILE);
+  g.sym = sym;
+  g.tiles_per_batch = sym ? g.tiles_m * (g.tiles_m + 1) / 2 : g.tiles_m * g.tiles_n;
+  g.num_kb = cdiv(k, 128);
+  g.debug_simt = g_starve_producers ? 0x100 : 0;
+  g.group = wide_group(k);
+  g.a_raw = a; g.b_raw = bt; g.status = status;
+  const long long tiles = (long long)g.tiles_per_batch * batch;
+  if (tiles > 0x7fffffffLL / 2) return fail(I8M_E_LIMIT, "%s: too many tiles", name);
+  if ((long long)g.num_kb * ((tiles + 1) / 1) > 0x7fffffffLL) return fail(I8M_E_LIMIT, "%s: too many K blocks", name);
+  CUtensorMap ma, mb;
+  if (int rc = make_operand_map(&ma, a, 1, k, m, batch)) return rc;
+  if (int rc = make_operand_map(&mb, bt, 1, k, n, batch)) return rc;
+  const unsigned grid = unsigned(std::min<long long>(tiles, sm_count()));
+  if constexpr (Epi::SPLIT_TAIL) {
+    if (g_bq_variant == 0) {
+      constexpr size_t SMEM = bq_split_smem_bytes<Epi>();
+      auto kernel = bq_split_kernel<Epi>;
+      static SmemAllowed allowed;
+      if (int rc = allow_smem(allowed, kernel, SMEM)) return rc;
+      launch(kernel, grid, BQS_THREADS, SMEM, stream, ma, mb, g, args);
+      LAUNCH_CHECK(name);
+      return 0;
+    }
+  }
+  const bool four = g_bq_variant == 2;
+  const int stages = four ? BQP_STAGES_ALT : BQP_STAGES;
+  const size_t SMEM = size_t(stages) * 2 * TILE_BYTES + sizeof(Ctrl) + 2 * BQP_MAX_KB * sizeof(float) +
+                      Epi::TSM_BYTES + 1024;
+  auto kernel = four ? bq_persistent_kernel<Epi, BQP_STAGES_ALT> : bq_persistent_kernel<Epi, BQP_STAGES>;
+  static SmemAllowed allowed[2];
+  if (int rc = allow_smem(allowed[four], kernel, SMEM)) return rc;
+  launch(kernel, grid, BQP_THREADS, SMEM, stream, ma, mb, g, args);
+  LAUNCH_CHECK(name);
+  return 0;
+}
+
+}  // namespace i8m

@@ -63,6 +63,7 @@ template <typename In>
 __global__ void __launch_bounds__(STATS_THREADS)
 stats_partial_kernel(const In* x, float* partial_sum, float* partial_max, long long count,
                      int chunks) {
+  pdl_wait();
   __shared__ float sh[8];
   const int b = blockIdx.y, chunk = blockIdx.x;
   const In* src = x + size_t(b) * count;
@@ -89,6 +90,7 @@ stats_partial_kernel(const In* x, float* partial_sum, float* partial_max, long l
 __global__ void __launch_bounds__(STATS_THREADS)
 stats_final_kernel(const float* partial_sum, const float* partial_max, float* norm, float* amax,
                    int chunks) {
+  pdl_wait();
   __shared__ float sh[8];
   const int b = blockIdx.x;
   float s = 0.f, mx = 0.f;
@@ -113,6 +115,7 @@ template <typename In>
 __global__ void __launch_bounds__(STATS_THREADS)
 stats_onepass_kernel(const In* x, float* sumsq, unsigned* amax_bits, unsigned* arrived, float* norm, float* amax,
                      long long count, int chunks) {
+  pdl_wait();
   __shared__ float sh[8];
   const int b = blockIdx.y, chunk = blockIdx.x;
   const In* src = x + size_t(b) * count;
@@ -145,6 +148,7 @@ stats_onepass_kernel(const In* x, float* sumsq, unsigned* amax_bits, unsigned* a
 // norm[b] <- max(norm[b], eps) / gain: folds an input gain into the dequantisation scale of the
 // grouped-cubic route (src/i8muon/_cutlass_cubic.py:38-40).
 __global__ void clamp_divide_kernel(float* norm, int batch, float eps, float gain) {
+  pdl_wait();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b < batch) norm[b] = __fdiv_rn(fmaxf(norm[b], eps), gain);
 }
@@ -156,6 +160,7 @@ template <typename In, typename E>
 __global__ void __launch_bounds__(256)
 normalize_kernel(const In* x, const float* norm, E* out, E* out_t, float* out_lo, float* out_t_lo,
                  int rows, int cols, int m, int n, int transpose, float eps) {
+  pdl_wait();
   __shared__ float tile[32][33];
   const int b = blockIdx.z;
   const float nb = norm ? norm[b] : 1.f;
@@ -227,6 +232,7 @@ template <typename In, typename E>
 __global__ void __launch_bounds__(256)
 normalize_vec_kernel(const In* x, const float* norm, E* out, E* out_t, int rows, int cols, int m, int n,
                      int transpose, float eps) {
+  pdl_wait();
   __shared__ __align__(16) uint8_t tile_t[64 * 128];   // [input column][input row] of E, swizzled
   const int b = blockIdx.z;
   const float nb = norm ? norm[b] : 1.f;
@@ -277,6 +283,7 @@ template <typename In, bool FP8>
 __global__ void __launch_bounds__(256)
 bq_quant_vec_kernel(const In* x, const float* norm, uint8_t* out, uint8_t* out_t, float* scale,
                     int rows, int cols, int m, int n, int transpose, float eps) {
+  pdl_wait();
   __shared__ float sh[8];
   __shared__ float s_mult;
   __shared__ __align__(16) uint8_t tile_t[128 * 128];   // [input column][input row] bytes, swizzled
@@ -347,6 +354,7 @@ template <typename In>
 __global__ void __launch_bounds__(256)
 input_quant_kernel(const In* x, const float* amax, const float* norm, int8_t* out, int8_t* out_t,
                    float* scale, int rows, int cols, int m, int n, int transpose, float eps) {
+  pdl_wait();
   __shared__ int8_t tile[32][33];
   const int b = blockIdx.z;
   const float mx = amax[b];
@@ -389,6 +397,7 @@ __global__ void __launch_bounds__(256)
 symmetric_quant_kernel(const In* input, const void* maximum, const float* orig_scale,
                        const float* orig_diag, int8_t* output, float* scale, float* diag, int m,
                        float c0, float c1, float c2) {
+  pdl_wait();
   __shared__ int8_t tile[32][33];
   const int b = blockIdx.y, pid = blockIdx.x;
   int tm = int((sqrtf(float(8 * pid + 1)) - 1.f) * 0.5f);
@@ -495,6 +504,7 @@ template <typename In>
 __global__ void __launch_bounds__(256)
 input_quant128_kernel(const In* x, const float* amax, const float* norm, int8_t* same, int8_t* other, float* scale,
                       int rows, int cols, float eps) {
+  pdl_wait();
   __shared__ uint32_t tile[128 * QT_PITCH];
   const int b = blockIdx.z;
   const float mx = amax[b];
@@ -527,6 +537,7 @@ input_quant128_kernel(const In* x, const float* amax, const float* norm, int8_t*
 __global__ void __launch_bounds__(256)
 output_quant128_kernel(const float* input, const float* maximum, int8_t* out, int8_t* out_t, float* scale, int m,
                        int n) {
+  pdl_wait();
   __shared__ uint32_t tile[128 * QT_PITCH];
   const int b = blockIdx.z;
   const float mx = maximum[b];
@@ -559,6 +570,7 @@ template <typename In, bool QUAD>
 __global__ void __launch_bounds__(256)
 symmetric_quant128_kernel(const In* input, const void* maximum, const float* orig_scale, const float* orig_diag,
                           int8_t* output, float* scale, float* diag, int m, float c0, float c1, float c2) {
+  pdl_wait();
   __shared__ uint32_t tile[128 * QT_PITCH];
   const int b = blockIdx.y, pid = blockIdx.x;
   int tm = int((sqrtf(float(8 * pid + 1)) - 1.f) * 0.5f);
@@ -627,6 +639,7 @@ symmetric_quant128_kernel(const In* input, const void* maximum, const float* ori
 template <typename E>
 __global__ void __launch_bounds__(256)
 diag_add_kernel(E* r, int batch, int m, int logical, float shift) {
+  pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (long long)batch * logical) return;
   const int b = int(i / logical), d = int(i - (long long)b * logical);
@@ -640,6 +653,7 @@ diag_add_kernel(E* r, int batch, int m, int logical, float shift) {
 __global__ void __launch_bounds__(256)
 output_quant_kernel(const float* input, const float* maximum, int8_t* out, int8_t* out_t,
                     float* scale, int m, int n) {
+  pdl_wait();
   __shared__ int8_t tile[32][33];
   const int b = blockIdx.z;
   const float mx = maximum[b];
@@ -676,6 +690,7 @@ template <typename In, bool FP8>
 __global__ void __launch_bounds__(256)
 bq_quant_kernel(const In* x, const float* norm, uint8_t* out, uint8_t* out_t, float* scale,
                 int rows, int cols, int m, int n, int transpose, float eps) {
+  pdl_wait();
   __shared__ float sh[8];
   __shared__ uint8_t qt[128][132];
   const int tmb = blockIdx.x, tnb = blockIdx.y, b = blockIdx.z;
@@ -756,6 +771,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 momentum_kernel(MomentumTable tab, T* update, long long numel, float w_buf, float mu,
                 int nesterov, float* partial_sum, float* partial_max, int chunks, int first_tensor) {
+  pdl_wait();
   __shared__ float sh[8];
   const int t = blockIdx.y;
   const T* g = static_cast<const T*>(tab.grad[t]);
@@ -830,7 +846,10 @@ momentum_kernel(MomentumTable tab, T* update, long long numel, float w_buf, floa
 template <typename P, typename U>
 __global__ void __launch_bounds__(256)
 apply_kernel(ApplyTable tab, const U* update, long long numel, int decay_mode, float decay,
-             float neg_lr) {
+             float neg_lr, const unsigned* status, unsigned* status_host) {
+  pdl_wait();
+  // the step's status word to the caller's pinned memory: one four-byte store instead of a copy in the stream
+  if (status_host && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *status_host = *status;
   const int t = blockIdx.y;
   P* p = static_cast<P*>(tab.param[t]);
   const U* u = update + size_t(t) * numel;
@@ -880,6 +899,7 @@ template <typename P, typename G>
 __global__ void __launch_bounds__(256)
 adamw_kernel(AdamTable tab, float decay, float beta1, float beta2, float eps, float step_size,
              float inv_bc2_sqrt) {
+  pdl_wait();
   const int t = blockIdx.y;
   P* p = static_cast<P*>(tab.param[t]);
   const G* g = static_cast<const G*>(tab.grad[t]);

@@ -22,6 +22,15 @@ class NativeError(RuntimeError):
     """A C-ABI call returned a negative code."""
 
 
+class GroupPlan(ctypes.Structure):
+    """``i8m_group_plan``: what stays the same from step to step for one shape group of the optimizer."""
+    _fields_ = [*[(name, c_int) for name in (
+        "count", "leading", "rows", "cols", "grad_dtype", "param_dtype", "route", "compute", "steps", "fp16_first",
+        "deterministic", "variants", "nesterov", "use_stats", "decay_mode")],
+        ("eps", c_float), ("buf_weight", c_float), ("mu", c_float), ("coeffs", POINTER(c_double)),
+        ("gram_order", c_char_p), ("status_device", c_void_p), ("status_host", c_void_p)]
+
+
 _P = c_void_p
 _SIGNATURES = {
     "i8m_version": (c_int, []),
@@ -63,6 +72,9 @@ _SIGNATURES = {
                              c_float, c_int, _P, _P]),
     "i8m_apply": (c_int, [POINTER(_P), c_int, _P, c_longlong, c_int, c_int, c_int, c_float,
                           c_float, _P]),
+    "i8m_group_bytes": (c_int, [POINTER(GroupPlan), POINTER(c_size_t)]),
+    "i8m_group_step": (c_int, [POINTER(GroupPlan), POINTER(_P), POINTER(_P), POINTER(_P), _P, c_size_t, c_float, c_float,
+                               _P]),
     "i8m_adamw": (c_int, [POINTER(_P), POINTER(_P), POINTER(_P), POINTER(_P), POINTER(c_longlong), c_int,
                           c_int, c_int, c_float, c_float, c_float, c_float, c_float, c_float, c_float, _P]),
 }
@@ -94,7 +106,9 @@ def check(code: int) -> None:
 
 
 def call(name: str, *args) -> None:
-    check(getattr(library(), name)(*args))
+    code = getattr(library(), name)(*args)
+    if code:
+        check(code)
 
 
 def pointer_array(pointers):
@@ -102,12 +116,19 @@ def pointer_array(pointers):
     return (_P * len(pointers))(*pointers)
 
 
+@lru_cache(maxsize=None)
 def torch_dtype_code(dtype) -> int:
     import torch
     try:
         return {torch.float32: F32, torch.float16: F16, torch.bfloat16: BF16}[dtype]
     except KeyError:
         raise ValueError("Input must be float32, float16 or bfloat16") from None
+
+
+def group_bytes(plan) -> int:
+    size = c_size_t(0)
+    call("i8m_group_bytes", ctypes.byref(plan), ctypes.byref(size))
+    return size.value
 
 
 def ns_workspace_bytes(route, batch, rows, cols, dtype, compute, steps, fp16_first) -> int:
