@@ -21,10 +21,10 @@ Differences that a caller can observe:
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import math
 import os
-from functools import lru_cache
 
 import torch
 
@@ -63,6 +63,19 @@ def check_status(device=None) -> None:
 _STATUS_HOST = {}
 
 
+def status_host(index: int) -> torch.Tensor:
+    """One int32 in pinned host memory per device, where the status word is copied to at the end of a step."""
+    host = _STATUS_HOST.get(index)
+    if host is None:
+        host = torch.zeros(1, dtype=torch.int32).pin_memory()
+        _STATUS_HOST[index] = host
+        _STATUS_VIEWS[index] = ctypes.c_int32.from_address(host.data_ptr())
+    return host
+
+
+_STATUS_VIEWS = {}   # the same words as ctypes integers: reading one is a plain load
+
+
 def post_status(device) -> None:
     """Queue a copy of the device's status word to pinned host memory on the current stream; nothing
     waits for it.  ``raise_if_reported`` looks at the copy once it has landed."""
@@ -71,32 +84,57 @@ def post_status(device) -> None:
     word = _STATUS_WORDS.get(index)
     if word is None or torch.cuda.is_current_stream_capturing():
         return
-    slot = _STATUS_HOST.get(index)
-    if slot is None:
-        slot = _STATUS_HOST[index] = (torch.zeros(1, dtype=torch.int32).pin_memory(), torch.cuda.Event())
-    host, event = slot
+    host = status_host(index)
     with torch.cuda.device(index):
         host.copy_(word, non_blocking=True)
-        event.record()
 
 
 def raise_if_reported() -> None:
-    """Raise if a status word copied by ``post_status`` has arrived and is not zero (no synchronisation)."""
-    for index, (host, event) in _STATUS_HOST.items():
-        if event.query() and int(host[0]) != 0:
-            code = int(host[0])
-            host.zero_()
+    """Raise if a status word copied to the host has arrived and is not zero (no synchronisation)."""
+    for index, view in _STATUS_VIEWS.items():
+        code = view.value
+        if code != 0:
+            torch.cuda.synchronize(index)   # copies still in flight land before the words are cleared
             _STATUS_WORDS[index].zero_()
+            view.value = 0
             raise native.NativeError(f"device-side wait timed out on cuda:{index}, status word 0x{code:x}; the "
                                      "results of the previous step are incomplete")
 
 
-def _coefficient_array(coeffs):
-    rows = [tuple(float(v) for v in row) for row in coeffs]
-    if not rows or any(len(row) != 3 for row in rows):
-        raise ValueError("Expected a nonempty list of (a, b, c) coefficients")
-    flat = [v for row in rows for v in row]
-    return (ctypes.c_double * len(flat))(*flat), len(rows)
+# raw handle of the current stream of a device; the public spelling builds a Stream object for every call
+raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (
+    lambda index: torch.cuda.current_stream(index).cuda_stream)
+_current_device = getattr(torch._C, "_cuda_getDevice", None) or torch.cuda.current_device
+_NO_SWITCH = contextlib.nullcontext()
+
+
+def on_device(index: int):
+    """Context in which CUDA device ``index`` is current (free when it already is)."""
+    return _NO_SWITCH if _current_device() == index else torch.cuda.device(index)
+
+
+def gram_order() -> str:
+    order = os.environ.get("I8MUON_GRAM_RESET", "00100")
+    if not order or order[0] != "0" or set(order) - {"0", "1"}:
+        raise ValueError("I8MUON_GRAM_RESET must be a binary string starting with 0")
+    return order
+
+
+_COEFFICIENT_ARRAYS = {}
+
+
+def coefficient_array(coeffs):
+    """The rows as a C array and their number; the arrays of recent schedules are kept."""
+    key = tuple([tuple(map(float, row)) for row in coeffs])
+    hit = _COEFFICIENT_ARRAYS.get(key)
+    if hit is None:
+        if not key or any(len(row) != 3 for row in key):
+            raise ValueError("Expected a nonempty list of (a, b, c) coefficients")
+        flat = [v for row in key for v in row]
+        hit = (ctypes.c_double * len(flat))(*flat), len(key)
+        if len(_COEFFICIENT_ARRAYS) < 256:
+            _COEFFICIENT_ARRAYS[key] = hit
+    return hit
 
 
 class CutlassNSInt8:
@@ -114,6 +152,8 @@ class CutlassNSInt8:
                 or any(v not in (0, 1, 2, 3, 4) for v in self.tiles.values())):
             raise ValueError("tiles accepts aat/square/update with values 0/1/2/3/4")
         self._routes = {}
+        self._specs = {}         # checked geometry and workspace size of the calls seen so far
+        self._group_plans = {}   # native plans of the optimizer's shape groups (optimizer.py)
         self._factory = KernelFactory(autotune)
 
     # ------------------------------------------------------------ routing
@@ -128,17 +168,22 @@ class CutlassNSInt8:
     # ------------------------------------------------------------- launch
     def _run(self, route, x, coeffs, eps, compute, alignment, spec_precision, fp16_first, out=None,
              deterministic=True, stats=None):
-        coeffs = DEFAULT_COEFFICIENTS if coeffs is None else coeffs
-        shape = x.shape
-        batch, rows, cols, *_ = matrix_spec(tuple(shape), x.dtype, x.device, spec_precision, alignment)
+        array, steps = coefficient_array(DEFAULT_COEFFICIENTS if coeffs is None else coeffs)
+        shape, device = x.shape, x.device
+        spec = (route, shape, x.dtype, device, compute, steps, alignment, spec_precision, bool(fp16_first))
+        known = self._specs.get(spec)
+        if known is None:
+            batch, rows, cols, *_ = matrix_spec(tuple(shape), x.dtype, device, spec_precision, alignment)
+            dtype = native.torch_dtype_code(x.dtype)
+            with on_device(device.index):
+                size = native.ns_workspace_bytes(route, batch, rows, cols, dtype, compute, steps, fp16_first)
+            known = batch, rows, cols, dtype, size, status_word(device).data_ptr()
+            if len(self._specs) < 1024:
+                self._specs[spec] = known
+        batch, rows, cols, dtype, size, status = known
         x = x.contiguous()
-        dtype = native.torch_dtype_code(x.dtype)
-        array, steps = _coefficient_array(coeffs)
-        order = os.environ.get("I8MUON_GRAM_RESET", "00100") if route == native.ROUTE_GRAM else None
-        if order is not None and (not order or order[0] != "0" or set(order) - {"0", "1"}):
-            raise ValueError("I8MUON_GRAM_RESET must be a binary string starting with 0")
-        with torch.cuda.device(x.device):
-            size = native.ns_workspace_bytes(route, batch, rows, cols, dtype, compute, steps, fp16_first)
+        order = gram_order().encode() if route == native.ROUTE_GRAM else None
+        with on_device(device.index):
             if out is None:
                 out = torch.empty_like(x)
             elif (out.shape != x.shape or out.dtype != x.dtype or out.device != x.device
@@ -149,16 +194,13 @@ class CutlassNSInt8:
                 raise ValueError("stats must be the FP32 partials that i8m_momentum left for x")
 
             def launch(variant):
-                workspace = torch.empty(size, dtype=torch.uint8, device=x.device)
+                workspace = torch.empty(size, dtype=torch.uint8, device=device)
                 native.call("i8m_ns_run", route, x.data_ptr(), out.data_ptr(), dtype, batch, rows, cols,
                             compute, array, steps, float(eps), int(bool(fp16_first)), int(bool(deterministic)),
-                            int(variant),
-                            order.encode() if order is not None else None,
-                            stats.data_ptr() if stats is not None else None, workspace.data_ptr(), size,
-                            status_word(x.device).data_ptr(), torch.cuda.current_stream().cuda_stream)
+                            int(variant), order, stats.data_ptr() if stats is not None else None,
+                            workspace.data_ptr(), size, status, raw_stream(device.index))
 
             variant = self.kernel_variants
-            key = (x.device.index, x.dtype, batch, rows, cols, route, compute, steps, bool(fp16_first))
             if route in (native.ROUTE_INT8, native.ROUTE_INT8_FACTORED) and self.tiles:
                 # explicit tiles take precedence over measurements, as in the reference
                 per_op = [0 if self.tiles.get(op, 4) == 4 else 2 for op in ("aat", "square", "update")]
@@ -166,6 +208,7 @@ class CutlassNSInt8:
             elif self._factory.autotune:
                 # per operation first (median of three graph replays, >= 2 % to replace the default), then the
                 # tuned call as a whole against the all-default call (>= 1 %), as the reference's factory does
+                key = (device.index, x.dtype, batch, rows, cols, route, compute, steps, bool(fp16_first))
                 tuned = 0
                 if route in (native.ROUTE_BQ_INT8, native.ROUTE_BQ_FP8):
                     tuned = self._factory.select("bq_gemm", key, tuple(range(native.variant_count("bq_gemm"))), 0, launch)
@@ -180,34 +223,43 @@ class CutlassNSInt8:
         # The workspace may be reused by later allocations on this stream only.
         return out.view(shape)
 
+    def call_spec(self, name: str, precision: str):
+        """(route, compute code, alignment, precision name of the geometry check, fp16_first) of the entry point
+        ``name`` at ``precision``."""
+        precision = normalize_precision(precision)
+        if name in ("_regular_prec", "_gram_prec"):
+            if precision not in _COMPUTE_CODES:
+                raise ValueError(f"Unsupported floating-point precision: {precision}")
+            route = native.ROUTE_FLOAT if name == "_regular_prec" else native.ROUTE_GRAM
+            return route, _COMPUTE_CODES[precision], 16, precision, False
+        if name == "_regular_i8":
+            return native.ROUTE_INT8, native.F16, 16, "int8", self.fp16_first
+        if precision in ("int8_bq", "int8"):
+            return native.ROUTE_BQ_INT8, native.F16, 128, "int8", self.fp16_first
+        if precision != "float8_e4m3fn":
+            raise ValueError(f"Unsupported block-quantised precision: {precision}")
+        return native.ROUTE_BQ_FP8, native.F16, 128, precision, False
+
+    def _call(self, name, x, coeffs, eps, deterministic, precision, out, stats):
+        route, compute, alignment, checked, fp16_first = self.call_spec(name, precision)
+        return self._run(route, x, coeffs, eps, compute, alignment, checked, fp16_first, out, deterministic, stats)
+
     # Every entry point takes the reference's arguments plus two keyword-only extras: ``out``, a caller-owned
     # tensor for the result (the sharded step lets NS write straight into its gather buffer), and ``stats``,
     # the statistics partials that the momentum kernel left for ``x`` (then no pass over ``x`` is needed
     # for its norm).
     def _regular_prec(self, x, coeffs=None, eps=1e-7, deterministic=True, precision="float16", *, out=None, stats=None):
         """FP32 / BF16 / FP16 regular NS (src/i8muon/_cutlass_prec.py:90-106)."""
-        precision = normalize_precision(precision)
-        if precision not in _COMPUTE_CODES:
-            raise ValueError(f"Unsupported floating-point precision: {precision}")
-        return self._run(native.ROUTE_FLOAT, x, coeffs, eps, _COMPUTE_CODES[precision], 16, precision, False, out,
-                         deterministic, stats)
+        return self._call("_regular_prec", x, coeffs, eps, deterministic, precision, out, stats)
 
     def _gram_prec(self, x, coeffs=None, eps=1e-7, deterministic=True, precision="float16", *, out=None, stats=None):
         """Gram-space NS with restarts given by I8MUON_GRAM_RESET (src/i8muon/_cutlass_prec.py:107-130)."""
-        precision = normalize_precision(precision)
-        if precision not in _COMPUTE_CODES:
-            raise ValueError(f"Unsupported floating-point precision: {precision}")
-        return self._run(native.ROUTE_GRAM, x, coeffs, eps, _COMPUTE_CODES[precision], 16, precision, False, out,
-                         deterministic, stats)
+        return self._call("_gram_prec", x, coeffs, eps, deterministic, precision, out, stats)
 
     def _regular_i8(self, x, coeffs=None, eps=1e-7, deterministic=True, precision="int8", *, block=False, out=None,
                     stats=None):
         """Global-scale INT8 NS, optionally after one FP16 iteration (src/i8muon/_cutlass.py:130-142)."""
-        if block:
-            return self._run(native.ROUTE_BQ_INT8, x, coeffs, eps, native.F16, 128, "int8", self.fp16_first, out,
-                             deterministic, stats)
-        return self._run(native.ROUTE_INT8, x, coeffs, eps, native.F16, 16, "int8", self.fp16_first, out, deterministic,
-                         stats)
+        return self._call("_regular_bq" if block else "_regular_i8", x, coeffs, eps, deterministic, "int8", out, stats)
 
     # ------------------------------------------------ opt-in polynomial entry points
     def _regular_i8_factored(self, X, factor_rows, eps=1e-7, deterministic=True, *, out=None):
@@ -237,13 +289,7 @@ class CutlassNSInt8:
                     stats=None):
         """128x128 block-quantised NS: INT8 honours fp16_first, E4M3 never does
         (src/i8muon/_cutlass.py:71-76)."""
-        precision = normalize_precision(precision)
-        if precision in ("int8_bq", "int8"):
-            return self._regular_i8(x, coeffs, eps, deterministic, "int8", block=True, out=out, stats=stats)
-        if precision != "float8_e4m3fn":
-            raise ValueError(f"Unsupported block-quantised precision: {precision}")
-        return self._run(native.ROUTE_BQ_FP8, x, coeffs, eps, native.F16, 128, precision, False, out, deterministic,
-                         stats)
+        return self._call("_regular_bq", x, coeffs, eps, deterministic, precision, out, stats)
 
 
-__all__ = ["CutlassNSInt8", "check_status", "status_word", "post_status", "raise_if_reported"]
+__all__ = ["CutlassNSInt8", "check_status", "status_word", "status_host", "post_status", "raise_if_reported"]

@@ -10,6 +10,8 @@ the device:
     stacked update tensor directly, and weight decay + the learning-rate-scaled
     update is one multi-tensor kernel; their roundings match the eager torch
     sequence of the reference;
+  * a group is one call into the library (momentum, Newton-Schulz, decay + update) over one block of scratch
+    memory; what does not change from step to step is kept in a plan per group;
   * with ``use_cuda_graph`` the whole Newton-Schulz call of a group (some thirty launches) is
     captured over a static update buffer and replayed; the two multi-tensor kernels run eagerly
     around it because they take the addresses of gradients and parameters and the learning
@@ -18,6 +20,7 @@ the device:
 from __future__ import annotations
 
 import contextlib
+import ctypes
 import os
 from typing import Optional
 
@@ -26,8 +29,9 @@ from torch import Tensor
 from torch.optim.optimizer import Optimizer, ParamsT
 
 from . import native
-from .coefficients import recommend_coefficients
-from .engine import CutlassNSInt8, post_status, raise_if_reported
+from .coefficients import DEFAULT_COEFFICIENTS, recommend_coefficients
+from .engine import (CutlassNSInt8, coefficient_array, gram_order, on_device, post_status, raise_if_reported, raw_stream,
+                     status_host, status_word)
 from .routing import (EPS, GRAM_ASPECT_THRESHOLD, adjust_lr, matrix_spec, normalize_precision,
                       validate_ns_device)
 
@@ -270,7 +274,7 @@ def _momentum(grads, bufs, update, w_buf, mu, nesterov, stats=None):
     native.call("i8m_momentum", native.pointer_array([g.data_ptr() for g in grads]),
                 native.pointer_array([b.data_ptr() for b in bufs]), len(grads), update.data_ptr(),
                 grads[0].numel(), native.torch_dtype_code(update.dtype), w_buf, mu, int(nesterov),
-                stats.data_ptr() if stats is not None else None, torch.cuda.current_stream().cuda_stream)
+                stats.data_ptr() if stats is not None else None, raw_stream(update.device.index))
 
 
 def muon_step(
@@ -317,11 +321,23 @@ def muon_step(
     groups: dict = {}
     for index, param in enumerate(params):
         grad, buf = grads[index], momentum_bufs[index]
-        if grad.shape != param.shape or buf.shape != grad.shape or buf.dtype != grad.dtype:
+        shape, gdtype = grad.shape, grad.dtype
+        if shape != param.shape or buf.shape != shape or buf.dtype != gdtype:
             raise ValueError("parameter, gradient and momentum buffer must agree in shape; "
                              "gradient and buffer in dtype")
-        key = (grad.device, grad.dtype, param.dtype, tuple(grad.shape))
-        groups.setdefault(key, []).append(index)
+        groups.setdefault((grad.device, gdtype, param.dtype, shape), []).append(index)
+
+    decay_mode = 0 if weight_decay == 0 else (2 if weight_decay_mode == "adjusted_lr" else 1)
+    decay = {0: 0.0, 2: weight_decay}.get(decay_mode, 1.0 - weight_decay if weight_decay_mode == "absolute"
+                                          else 1.0 - lr * weight_decay)
+    # this library's own engine with its default kernel selection: a group is one native call
+    own_engine = type(ns_engine) is CutlassNSInt8
+    whole_groups = own_engine and not use_cuda_graph and not ns_engine.autotune and not ns_engine.tiles
+    if whole_groups:
+        array, steps = coefficient_array(DEFAULT_COEFFICIENTS if ns_coefficients is None else ns_coefficients)
+        settings = (ctypes.addressof(array), steps, eps, deterministic, mu, mu2, nesterov, decay_mode,
+                    ns_engine.fp16_first, ns_engine.kernel_variants)
+    posted = set()           # devices whose status word the groups' own update kernels have posted
 
     for (device, gdtype, pdtype, shape), members in groups.items():
         M, N = shape[-2], shape[-1]
@@ -333,25 +349,38 @@ def muon_step(
         # this library's engine takes the statistics partials that the momentum kernel leaves; a foreign
         # engine with the reference's call convention does not
         takes_stats = isinstance(ns_engine, CutlassNSInt8) and deterministic and len(shape) == 2
-        per_tensor = 1
-        for d in shape:
-            per_tensor *= d
+        per_tensor = shape.numel()
         leading = per_tensor // (M * N)
         chunk = max(1, min(len(members), MAX_GROUP_BYTES // max(1, per_tensor * grads[members[0]].element_size()),
                            65535 // max(1, leading)))
-        with torch.cuda.device(device):
+        with on_device(device.index):
             for first in range(0, len(members), chunk):
                 part = members[first:first + chunk]
-                g_list = [grads[i] if grads[i].is_contiguous() else grads[i].contiguous() for i in part]
-                b_list, p_list, copy_back = [], [], []
+                g_list, b_list, p_list, copy_back = [], [], [], []
                 for i in part:
-                    b, p = momentum_bufs[i], params[i]
+                    g, b, p = grads[i], momentum_bufs[i], params[i]
+                    if not g.is_contiguous():
+                        g = g.contiguous()
                     if not b.is_contiguous():
                         c = b.contiguous(); copy_back.append((b, c)); b = c
                     if not p.is_contiguous():
                         c = p.contiguous(); copy_back.append((p, c)); p = c
-                    b_list.append(b); p_list.append(p)
+                    g_list.append(g); b_list.append(b); p_list.append(p)
                 count = len(part)
+                if whole_groups:
+                    plan, block_bytes = _group_plan(ns_engine, ns_fn.__name__, actual, settings, array, device, gdtype,
+                                                    pdtype, shape, count, leading, takes_stats)
+                    if callable(adjust_lr_fn):
+                        adjusted = adjust_lr(lr, adjust_lr_fn, shape)
+                    pointers = _P_ARRAYS.get(count) or _P_ARRAYS.setdefault(count, ctypes.c_void_p * count)
+                    block = torch.empty(block_bytes, dtype=torch.uint8, device=device)
+                    native.call("i8m_group_step", plan, pointers(*[g.data_ptr() for g in g_list]),
+                                pointers(*[b.data_ptr() for b in b_list]), pointers(*[p.data_ptr() for p in p_list]),
+                                block.data_ptr(), block_bytes, decay, -_as_float(adjusted), raw_stream(device.index))
+                    posted.add(device)
+                    for original, contiguous in copy_back:
+                        original.copy_(contiguous)
+                    continue
                 update = None
                 if use_cuda_graph:
                     key = _graph_key(ns_fn, g_list[0], count, actual, ns_coefficients, eps, deterministic, ns_engine)
@@ -386,23 +415,42 @@ def muon_step(
 
                 if callable(adjust_lr_fn):
                     adjusted = adjust_lr(lr, adjust_lr_fn, shape)
-                adjusted = _as_float(adjusted)
-                if weight_decay == 0:
-                    mode, decay = 0, 0.0
-                elif weight_decay_mode == "adjusted_lr":
-                    mode, decay = 2, weight_decay
-                elif weight_decay_mode == "absolute":
-                    mode, decay = 1, 1.0 - weight_decay
-                else:
-                    mode, decay = 1, 1.0 - lr * weight_decay
                 native.call("i8m_apply", native.pointer_array([p.data_ptr() for p in p_list]), count,
                             ortho.data_ptr(), per_tensor, native.torch_dtype_code(pdtype),
-                            native.torch_dtype_code(gdtype), mode, decay, -adjusted,
-                            torch.cuda.current_stream().cuda_stream)
+                            native.torch_dtype_code(gdtype), decay_mode, decay, -_as_float(adjusted),
+                            raw_stream(device.index))
                 for original, contiguous in copy_back:
                     original.copy_(contiguous)
-    for device in {g.device for g in grads if g.device.type == "cuda"}:
-        post_status(device)
+    for device in {key[0] for key in groups}:
+        if device.type == "cuda" and device not in posted:
+            post_status(device)
+
+
+_P_ARRAYS: dict = {}      # count -> ctypes array type
+MAX_GROUP_PLANS = 512
+
+
+def _group_plan(engine, name, precision, settings, array, device, gdtype, pdtype, shape, count, leading, takes_stats):
+    """The native plan of one shape group and the bytes of scratch memory it needs (kept per engine)."""
+    order = gram_order() if name == "_gram_prec" else None
+    key = (name, precision, settings, device, gdtype, pdtype, shape, count, takes_stats, order)
+    hit = engine._group_plans.get(key)
+    if hit is None:
+        route, compute, alignment, checked, fp16_first = engine.call_spec(name, precision)
+        matrix_spec((count, *shape), gdtype, device, checked, alignment)
+        _, steps, eps, deterministic, mu, mu2, nesterov, decay_mode, _, variants = settings
+        plan = native.GroupPlan(
+            count=count, leading=leading, rows=shape[-2], cols=shape[-1], grad_dtype=native.torch_dtype_code(gdtype),
+            param_dtype=native.torch_dtype_code(pdtype), route=route, compute=compute, steps=steps,
+            fp16_first=int(bool(fp16_first)), deterministic=int(bool(deterministic)), variants=variants,
+            nesterov=int(nesterov), use_stats=int(takes_stats), decay_mode=decay_mode, eps=float(eps),
+            buf_weight=1.0 - mu2, mu=mu, coeffs=array, gram_order=order.encode() if order else None,
+            status_device=status_word(device).data_ptr(), status_host=status_host(device.index).data_ptr())
+        hit = ctypes.byref(plan), native.group_bytes(plan), plan, array   # the array lives as long as the plan
+        if len(engine._group_plans) >= MAX_GROUP_PLANS:
+            engine._group_plans.clear()
+        engine._group_plans[key] = hit
+    return hit[0], hit[1]
 
 
 def native_step_ops(ns_engine: CutlassNSInt8, *, lr, weight_decay, momentum, ns_coefficients, eps=EPS,
