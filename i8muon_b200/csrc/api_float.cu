@@ -1,5 +1,6 @@
 // C ABI: floating-point products.
 #include "launch_gemm.cuh"
+#include "drivers.cuh"
 #include "epi_float.cuh"
 #include "epi_float_bq.cuh"
 
@@ -8,82 +9,75 @@ using namespace i8m;
 namespace {
 
 template <typename E>
-int float_gemm_typed(const void* left, const void* left_lo, const void* right_t,
-                     const void* right_t_lo, void* out, void* out_t, void* out_lo, void* out_t_lo,
-                     int mode, int batch, int m, int n, int k, int lm, int ln, int symmetric,
-                     int final, int transpose, int out_dtype, float ca, float cb, float cc,
-                     unsigned* status, cudaStream_t stream) {
+int float_gemm_typed(const FloatGemm& f) {
   FloatArgs a;
-  a.out = out; a.out_t = out_t; a.out_lo = out_lo; a.out_t_lo = out_t_lo;
-  a.src = left; a.src_lo = left_lo;
-  a.out_dtype = out_dtype; a.transpose = transpose;
-  a.ca = ca; a.cb = cb; a.cc = cc;
-  a.amax = final ? g_final_amax : nullptr;
-  if (mode == 1) {
-    if (final) return fail(I8M_E_ARGUMENT, "float_gemm: the polynomial mode has no final variant");
-    if (k != n) return fail(I8M_E_ARGUMENT, "float_gemm: polynomial mode needs a square left operand");
-    return launch_gemm<EpiFloat<E, MODE_QUAD>>(left, left_lo, right_t, right_t_lo, batch, m, n, k,
-                                               lm, ln, symmetric, status, a, stream, "float_gemm(poly)");
+  a.out = f.out; a.out_t = f.out_t; a.out_lo = f.out_lo; a.out_t_lo = f.out_t_lo;
+  a.src = f.left; a.src_lo = f.left_lo;
+  a.out_dtype = f.out_dtype; a.transpose = f.transpose;
+  a.ca = f.ca; a.cb = f.cb; a.cc = f.cc;
+  a.amax = f.final ? f.amax : nullptr;
+  GemmCall g;
+  g.a = f.left; g.a_lo = f.left_lo; g.b = f.right; g.b_lo = f.right_lo; g.a_mn = f.left_mn; g.b_mn = f.right_mn;
+  g.batch = f.batch; g.m = f.m; g.n = f.n; g.k = f.k; g.lm = f.lm; g.ln = f.ln;
+  g.sym = f.final ? 0 : f.symmetric; g.status = f.status; g.stream = f.stream;
+  if (f.mode == 1) {
+    if (f.final) return fail(I8M_E_ARGUMENT, "float_gemm: the polynomial mode has no final variant");
+    if (f.k != f.n) return fail(I8M_E_ARGUMENT, "float_gemm: polynomial mode needs a square left operand");
+    return launch_gemm<EpiFloat<E, MODE_QUAD>>(g, a, "float_gemm(poly)");
   }
-  if (final) {
-    if (!float_dtype_ok(out_dtype)) return fail(I8M_E_ARGUMENT, "float_gemm: bad out_dtype %d", out_dtype);
-    return launch_gemm<EpiFloat<E, MODE_FINAL>>(left, left_lo, right_t, right_t_lo, batch, m, n, k,
-                                                lm, ln, 0, status, a, stream, "float_gemm(final)");
+  if (f.final) {
+    if (!float_dtype_ok(f.out_dtype)) return fail(I8M_E_ARGUMENT, "float_gemm: bad out_dtype %d", f.out_dtype);
+    return launch_gemm<EpiFloat<E, MODE_FINAL>>(g, a, "float_gemm(final)");
   }
-  return launch_gemm<EpiFloat<E, MODE_PLAIN>>(left, left_lo, right_t, right_t_lo, batch, m, n, k, lm,
-                                              ln, symmetric, status, a, stream, "float_gemm");
+  return launch_gemm<EpiFloat<E, MODE_PLAIN>>(g, a, "float_gemm");
 }
-
 }  // namespace
 
+int i8m::float_gemm(const FloatGemm& f) {
+  if (!f.out || (f.mode != 0 && f.mode != 1)) return fail(I8M_E_ARGUMENT, "float_gemm: bad argument");
+  if (f.compute == I8M_F32) return float_gemm_typed<float>(f);
+  if (f.compute == I8M_F16) return float_gemm_typed<__half>(f);
+  if (f.compute == I8M_BF16) return float_gemm_typed<__nv_bfloat16>(f);
+  return fail(I8M_E_ARGUMENT, "float_gemm: bad compute dtype %d", f.compute);
+}
 extern "C" int i8m_float_gemm(const void* left, const void* left_lo, const void* right_t,
                               const void* right_t_lo, void* out, void* out_t, void* out_lo,
                               void* out_t_lo, int compute, int mode, int batch, int m, int n, int k,
                               int lm, int ln, int symmetric, int final, int transpose,
                               int out_dtype, float ca, float cb, float cc, uint32_t* status,
                               i8m_stream_t stream) {
-  if (!out || (mode != 0 && mode != 1)) return fail(I8M_E_ARGUMENT, "float_gemm: bad argument");
-  if (compute == I8M_F32)
-    return float_gemm_typed<float>(left, left_lo, right_t, right_t_lo, out, out_t, out_lo, out_t_lo,
-                                   mode, batch, m, n, k, lm, ln, symmetric, final, transpose,
-                                   out_dtype, ca, cb, cc, status, S(stream));
-  if (compute == I8M_F16)
-    return float_gemm_typed<__half>(left, left_lo, right_t, right_t_lo, out, out_t, out_lo, out_t_lo,
-                                    mode, batch, m, n, k, lm, ln, symmetric, final, transpose,
-                                    out_dtype, ca, cb, cc, status, S(stream));
-  if (compute == I8M_BF16)
-    return float_gemm_typed<__nv_bfloat16>(left, left_lo, right_t, right_t_lo, out, out_t, out_lo,
-                                           out_t_lo, mode, batch, m, n, k, lm, ln, symmetric, final,
-                                           transpose, out_dtype, ca, cb, cc, status, S(stream));
-  return fail(I8M_E_ARGUMENT, "float_gemm: bad compute dtype %d", compute);
+  return float_gemm(FloatGemm{left, left_lo, right_t, right_t_lo, out, out_t, out_lo, out_t_lo, compute, mode, batch, m, n, k,
+                              lm, ln, symmetric, final, transpose, out_dtype, 0, 0, ca, cb, cc, nullptr, status, S(stream)});
 }
 
 // FP16 / BF16 product whose result leaves as block-quantised INT8 operands (the end of the FP16 first
 // iteration of an fp16-first INT8-BQ call): persistent kernel only.
 template <typename E>
-static int float_gemm_to_bq_typed(const void* left, const void* right_t, const FloatToBqArgs& args, int batch, int m,
-                                  int n, int k, int lm, int ln, unsigned* status, cudaStream_t stream) {
+static int float_gemm_to_bq_typed(const void* left, const void* right, int right_mn, const FloatToBqArgs& args, int batch,
+                                  int m, int n, int k, int lm, int ln, unsigned* status, cudaStream_t stream) {
   using Epi = EpiFloatToBq<E>;
-  GemmGeom g;
+  GemmGeom g{};
   g.batch = batch; g.m = m; g.n = n; g.k = k; g.lm = lm; g.ln = ln;
   g.tiles_m = cdiv(m, TILE); g.tiles_n = cdiv(n, TILE);
   g.sym = 0;
   g.tiles_per_batch = g.tiles_m * g.tiles_n;
   g.num_kb = cdiv((long long)k * 2, 128);
-  g.debug_simt = 0;
+  g.b_mn = right_mn;
   g.group = wide_group(2LL * k);
-  g.a_raw = left; g.b_raw = right_t; g.status = status;
+  g.a_raw = left; g.b_raw = right; g.status = status;
   const long long blocks = (long long)g.tiles_per_batch * batch;
   if (blocks > 0x7fffffffLL) return fail(I8M_E_LIMIT, "float_gemm_to_bq: too many tiles");
   CUtensorMap ma, mb;
   if (int rc = make_operand_map(&ma, left, 2, k, m, batch)) return rc;
-  if (int rc = make_operand_map(&mb, right_t, 2, k, n, batch)) return rc;
+  if (int rc = make_operand_map(&mb, right, 2, k, n, batch, right_mn)) return rc;
   if (g_wholek_variant == 0) {
     constexpr size_t WSMEM = wholek_wide_smem_bytes<Epi>();
     auto wk = wholek_wide_kernel<Epi>;
     static SmemAllowed allowed;
     if (int rc = allow_smem(allowed, wk, WSMEM)) return rc;
-    const long long units = (long long)wide_units_per_batch(g.tiles_m, g.tiles_n, 0) * batch;
+    const long long pairs = (long long)wide_units_per_batch(g.tiles_m, g.tiles_n, 0) * batch;
+    g.narrow = narrow_units(blocks, pairs, g.num_kb, sm_count());
+    const long long units = g.narrow ? blocks : pairs;
     launch(wk, unsigned(std::min<long long>(units, sm_count())), WKW_THREADS, WSMEM, stream, ma, mb, g, args);
     LAUNCH_CHECK("float_gemm_to_bq");
     return 0;
@@ -98,10 +92,10 @@ static int float_gemm_to_bq_typed(const void* left, const void* right_t, const F
   return 0;
 }
 
-extern "C" int i8m_float_gemm_to_bq(const void* left, const void* right_t, void* q, void* q_t, float* scale,
-                                    int compute, int user_dtype, int batch, int m, int n, int k, int lm, int ln,
-                                    int lp, int hp, uint32_t* status, i8m_stream_t stream) {
-  if (!left || !right_t || !q || !q_t || !scale || !status) return fail(I8M_E_ARGUMENT, "float_gemm_to_bq: null pointer");
+int i8m::float_gemm_to_bq(const void* left, const void* right, int right_mn, void* q, void* q_t, float* scale, int compute,
+                          int user_dtype, int batch, int m, int n, int k, int lm, int ln, int lp, int hp, unsigned* status,
+                          cudaStream_t stream) {
+  if (!left || !right || !q || !q_t || !scale || !status) return fail(I8M_E_ARGUMENT, "float_gemm_to_bq: null pointer");
   if (batch < 1 || m < 1 || n < 1 || k < 1 || lm < 1 || ln < 1 || lm > m || ln > n)
     return fail(I8M_E_ARGUMENT, "float_gemm_to_bq: bad extents");
   if (lp % 128 || hp % 128 || lp < m || hp < n || cdiv(lp, 128) != cdiv(m, 128) || cdiv(hp, 128) != cdiv(n, 128))
@@ -111,8 +105,14 @@ extern "C" int i8m_float_gemm_to_bq(const void* left, const void* right_t, void*
   a.q = static_cast<uint8_t*>(q); a.qt = static_cast<uint8_t*>(q_t); a.scale = scale;
   a.lp = lp; a.hp = hp; a.user_dtype = user_dtype;
   if (compute == I8M_F16)
-    return float_gemm_to_bq_typed<__half>(left, right_t, a, batch, m, n, k, lm, ln, status, S(stream));
+    return float_gemm_to_bq_typed<__half>(left, right, right_mn, a, batch, m, n, k, lm, ln, status, stream);
   if (compute == I8M_BF16)
-    return float_gemm_to_bq_typed<__nv_bfloat16>(left, right_t, a, batch, m, n, k, lm, ln, status, S(stream));
+    return float_gemm_to_bq_typed<__nv_bfloat16>(left, right, right_mn, a, batch, m, n, k, lm, ln, status, stream);
   return fail(I8M_E_ARGUMENT, "float_gemm_to_bq: compute must be a 16-bit type");
+}
+extern "C" int i8m_float_gemm_to_bq(const void* left, const void* right_t, void* q, void* q_t, float* scale,
+                                    int compute, int user_dtype, int batch, int m, int n, int k, int lm, int ln,
+                                    int lp, int hp, uint32_t* status, i8m_stream_t stream) {
+  return float_gemm_to_bq(left, right_t, 0, q, q_t, scale, compute, user_dtype, batch, m, n, k, lm, ln, lp, hp, status,
+                          S(stream));
 }

@@ -14,27 +14,26 @@ extern "C" int i8m_i8_gemm(int mode, const int8_t* a, const int8_t* b_t, const i
   g.out = out; g.maximum = maximum; g.a_scale = a_scale; g.b_scale = b_scale; g.diag = diag;
   g.row_b = row_b; g.alpha = alpha; g.beta = beta; g.out_dtype = out_dtype; g.transpose = transpose;
   g.gain = alpha; g.use_gain = mode == 4;
+  GemmCall c;
+  c.a = a; c.b = b_t; c.batch = batch; c.m = m; c.n = n; c.k = k; c.lm = lm; c.ln = ln;
+  c.sym = mode < 2; c.status = status; c.stream = S(stream);
   if (mode == 4) mode = 2;   // update whose right-hand scale is multiplied by alpha
   if (mode == 0) {
     if (!maximum) return fail(I8M_E_ARGUMENT, "i8_gemm: gram needs a maximum slot");
-    return launch_gemm<EpiI8<I8_GRAM>>(a, nullptr, b_t, nullptr, batch, m, n, k, lm, ln, 1, status, g,
-                                       S(stream), "i8_gemm(gram)");
+    return launch_gemm<EpiI8<I8_GRAM>>(c, g, "i8_gemm(gram)");
   }
   if (mode == 1) {
     if (!maximum || !a_scale || !diag) return fail(I8M_E_ARGUMENT, "i8_gemm: square needs scale, diag, maximum");
-    return launch_gemm<EpiI8<I8_SQUARE>>(a, nullptr, b_t, nullptr, batch, m, n, k, lm, ln, 1, status,
-                                         g, S(stream), "i8_gemm(square)");
+    return launch_gemm<EpiI8<I8_SQUARE>>(c, g, "i8_gemm(square)");
   }
   if (mode == 2) {
     if (!a_scale || !b_scale || !diag || !row_b) return fail(I8M_E_ARGUMENT, "i8_gemm: update needs scales, diag, row_b");
     if (final) {
       if (!float_dtype_ok(out_dtype)) return fail(I8M_E_ARGUMENT, "i8_gemm: bad out_dtype");
-      return launch_gemm<EpiI8<I8_UPDATE_FINAL>>(a, nullptr, b_t, nullptr, batch, m, n, k, lm, ln, 0,
-                                                 status, g, S(stream), "i8_gemm(final update)");
+      return launch_gemm<EpiI8<I8_UPDATE_FINAL>>(c, g, "i8_gemm(final update)");
     }
     if (!maximum) return fail(I8M_E_ARGUMENT, "i8_gemm: update needs a maximum slot");
-    return launch_gemm<EpiI8<I8_UPDATE>>(a, nullptr, b_t, nullptr, batch, m, n, k, lm, ln, 0, status, g,
-                                         S(stream), "i8_gemm(update)");
+    return launch_gemm<EpiI8<I8_UPDATE>>(c, g, "i8_gemm(update)");
   }
   return fail(I8M_E_ARGUMENT, "i8_gemm: bad mode %d", mode);
 }

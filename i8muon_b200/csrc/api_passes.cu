@@ -115,6 +115,26 @@ extern "C" int i8m_normalize(const void* x, int in_dtype, const float* norm, voi
                                 static_cast<const In*>(x), norm, static_cast<E*>(a),           \
                                 static_cast<E*>(a_t), static_cast<float*>(a_lo),               \
                                 static_cast<float*>(a_t_lo), rows, cols, lp, hp, transpose, eps)))
+  if (a_t == nullptr && !transpose && compute != I8M_F32 && hp % 8 == 0 && (reinterpret_cast<uintptr_t>(a) & 15u) == 0) {
+    // no transposed copy: a plain element-wise pass
+    const bool vectors = (size_t(cols) * dtype_size(in_dtype)) % 16 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
+    const long long groups = (long long)lp * (hp / 8);
+    const dim3 rgrid(unsigned(std::min<long long>(cdiv(groups, 256), std::max(1, 148 * 32 / batch))), batch);
+#define NORM_ROWS(In, E)                                                                                              \
+  do {                                                                                                                \
+    if (vectors)                                                                                                      \
+      launch(normalize_rows_kernel<In, E, true>, rgrid, 256, 0, S(stream), static_cast<const In*>(x), norm,           \
+             static_cast<E*>(a), rows, cols, lp, hp, eps);                                                            \
+    else                                                                                                              \
+      launch(normalize_rows_kernel<In, E, false>, rgrid, 256, 0, S(stream), static_cast<const In*>(x), norm,          \
+             static_cast<E*>(a), rows, cols, lp, hp, eps);                                                            \
+  } while (0)
+    if (compute == I8M_F16) DISPATCH_IN(in_dtype, In, NORM_ROWS(In, __half));
+    else DISPATCH_IN(in_dtype, In, NORM_ROWS(In, __nv_bfloat16));
+#undef NORM_ROWS
+    LAUNCH_CHECK("normalize");
+    return 0;
+  }
   // 16-bit out, rows of whole 16-byte vectors: the vectorised kernel
   const bool vec = compute != I8M_F32 && cols % 8 == 0 && lp % 8 == 0 && hp % 8 == 0 &&
                    ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(a) |

@@ -1,8 +1,25 @@
-// Passes that only the whole-call drivers launch.
+// What the whole-call drivers launch beyond the C ABI's own entry points.
 #pragma once
 #include <cuda_runtime.h>
 
 namespace i8m {
+// out = left * right^T with the epilogues of i8m_float_gemm; an operand with its _mn flag set is stored with its
+// rows along K, (batch, k, m) or (batch, k, n), instead of (batch, m, k) or (batch, n, k).
+struct FloatGemm {
+  const void *left, *left_lo, *right, *right_lo;
+  void *out, *out_t, *out_lo, *out_t_lo;
+  int compute, mode, batch, m, n, k, lm, ln;
+  int symmetric, final, transpose, out_dtype;
+  int left_mn, right_mn;
+  float ca, cb, cc;
+  float* amax;     // final products, optional: [batch] maximum magnitude of the stored values (zeroed by the caller)
+  unsigned* status;
+  cudaStream_t stream;
+};
+int float_gemm(const FloatGemm& g);
+int float_gemm_to_bq(const void* left, const void* right, int right_mn, void* q, void* q_t, float* scale, int compute,
+                     int user_dtype, int batch, int m, int n, int k, int lm, int ln, int lp, int hp, unsigned* status,
+                     cudaStream_t stream);
 // final fold of per-chunk partials (i8m_stats layout) into norm[b] and amax[b]; either may be null
 int fold_stats(const float* partials, int batch, long long count, float* norm, float* amax, cudaStream_t stream);
 // r[b][i][i] += shift for i < logical, r (batch, m, m) in a 16-bit compute type

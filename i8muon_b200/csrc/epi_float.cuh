@@ -121,16 +121,18 @@ struct EpiFloat {
   static constexpr uint32_t IDESC = make_idesc(1u, FMT, FMT, TILE, TILE);
   using Args = FloatArgs;
 
-  // Fast path of the 16-bit types for a tile that lies inside the logical extent: packed
-  // conversions, 16-byte loads and stores only, the transposed copy through a 32 x 32 transpose in
-  // the warp's own shared-memory patch (64 contiguous bytes per lane instead of 32 scattered
-  // 2-byte stores).  Same roundings and the same un-fused arithmetic as the general path below.
+  // Fast path of the 16-bit types: packed conversions and coalesced accesses only, the transposed copy through a
+  // 32 x 32 transpose in the warp's own shared-memory patch (64 contiguous bytes per lane instead of 32 scattered
+  // 2-byte stores).  Blocks on the edge of a matrix go the same way, clipped to its extents and with zeros beyond the
+  // logical ones: on the general path below an edge tile took four times as long as an inner one and set the time of
+  // the whole product (BF16 square of a 1531 x 1531 matrix 44 us; see the figures at the launcher).  Same roundings and the
+  // same un-fused arithmetic as the general path, which serves the kernels without patches.
   static __device__ __forceinline__ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
   static __device__ __forceinline__ bool fast_ok(const GemmGeom& g, const Args& a, const TileCtx& t) {
-    if (t.wsm == nullptr || t.row0 + TILE > g.lm || t.col0 + TILE > g.ln) return false;
+    if (t.wsm == nullptr) return false;
     if constexpr (MODE == MODE_FINAL) {
-      if (a.out_dtype != DT_F16 && a.out_dtype != DT_BF16) return false;
-      return aligned16(a.out) && ((a.transpose ? g.lm : g.ln) & 7) == 0;
+      if (!a.transpose) return true;
+      return a.out_dtype != DT_F32 && aligned16(a.out) && (g.lm & 7) == 0 && t.row0 + TILE <= g.lm && t.col0 + TILE <= g.ln;
     } else {
       bool ok = aligned16(a.out) && (g.n & 7) == 0 && (g.m & 7) == 0 && (a.out_t == nullptr || aligned16(a.out_t));
       if constexpr (MODE == MODE_QUAD) ok = ok && aligned16(a.src) && (g.k & 7) == 0;
@@ -138,7 +140,46 @@ struct EpiFloat {
     }
   }
 
-  template <class Acc>
+  // The un-padded result in the caller's dtype, row-major, from 32 packed pairs p (this lane's row of the block).
+  static __device__ __forceinline__ void store_final(const GemmGeom& g, const Args& a, const TileCtx& t, const WarpPatch& wp,
+                                                     const uint32_t (&p)[16], int wrow0, int colb, const BlockClip clip) {
+    const size_t first = (size_t(t.b) * g.lm + wrow0) * g.ln + colb;
+    if (a.out_dtype == DT_F32) {
+      float* out = static_cast<float*>(a.out) + first;
+      const bool vectors = aligned16(a.out) && (g.ln & 3) == 0;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        uint32_t w[16];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const float2 f = unpack2<E>(p[8 * h + k]);
+          w[2 * k] = __float_as_uint(f.x); w[2 * k + 1] = __float_as_uint(f.y);
+        }
+        wp.write_own_row(w);
+        __syncwarp();
+        const int cols = clip.cols - 16 * h;
+        if (vectors) store_block_rows(wp, reinterpret_cast<uint8_t*>(out + 16 * h), size_t(g.ln) * 4, clip.rows, cols * 4);
+        else store_block_elements32(wp, reinterpret_cast<uint32_t*>(out + 16 * h), size_t(g.ln), clip.rows, cols);
+        __syncwarp();
+      }
+      return;
+    }
+    wp.write_own_row(p);
+    __syncwarp();
+    uint16_t* out = static_cast<uint16_t*>(a.out) + first;
+    if (a.transpose)
+      store_block_columns16(wp, reinterpret_cast<uint8_t*>(static_cast<uint16_t*>(a.out) + (size_t(t.b) * g.ln + colb) * g.lm + wrow0),
+                            size_t(g.lm) * 2);
+    else if (aligned16(a.out) && (g.ln & 7) == 0)
+      store_block_rows(wp, reinterpret_cast<uint8_t*>(out), size_t(g.ln) * 2, clip.rows, clip.cols * 2);
+    else
+      store_block_elements16(wp, out, size_t(g.ln), clip.rows, clip.cols);
+    __syncwarp();
+  }
+
+  // EDGE: the tile reaches beyond the logical extents.  Inner tiles carry no clipping code (it cost 5 % of a call over
+  // 768-wide matrices, whose products are mostly epilogue).
+  template <bool EDGE, class Acc>
   static __device__ __forceinline__ void run_fast(const GemmGeom& g, const Args& a, const TileCtx& t,
                                                   const Acc& acc) {
     const bool diag_tile = g.sym && t.tm == t.tn;
@@ -151,12 +192,15 @@ struct EpiFloat {
       uint32_t v[32];
       acc.load(c, v);
       const int colb = t.col0 + c * 32;
+      if (EDGE && (colb >= g.n || wrow0 >= g.m)) continue;       // uniform over the warp
+      // what the padded matrix holds of this block
+      const BlockClip held = EDGE ? BlockClip{g.m - wrow0, g.n - colb} : BlockClip{32, 32};
       uint32_t p[16];
       if constexpr (MODE == MODE_QUAD) {
         // the left operand's block R[wrow0 .. + 31][colb .. + 31]: coalesced into the patch, then one row per lane
         load_block_rows(wp, reinterpret_cast<const uint8_t*>(static_cast<const E*>(a.src) +
                                                              (size_t(t.b) * g.m + wrow0) * g.k + colb),
-                        size_t(g.k) * 2);
+                        size_t(g.k) * 2, held.rows, 2 * held.cols);
         __syncwarp();
         uint32_t rr[16];
         wp.read_own_row(rr);
@@ -175,9 +219,14 @@ struct EpiFloat {
 #pragma unroll
         for (int k = 0; k < 16; ++k) p[k] = pack2<E>(__uint_as_float(v[2 * k]), __uint_as_float(v[2 * k + 1]));
       }
+      if (EDGE) {   // padding is zero
+        const int cols = t.row < g.lm ? g.ln - colb : 0;
+#pragma unroll
+        for (int k = 0; k < 16; ++k) p[k] &= (2 * k < cols ? 0xffffu : 0u) | (2 * k + 1 < cols ? 0xffff0000u : 0u);
+      }
       if constexpr (MODE == MODE_FINAL) {
         // E -> the user's 16-bit type (a second rounding when they differ, as in the general path)
-        if (a.out_dtype != E_CODE) {
+        if (a.out_dtype != E_CODE && a.out_dtype != DT_F32) {
 #pragma unroll
           for (int k = 0; k < 16; ++k) {
             const float2 f = unpack2<E>(p[k]);
@@ -187,30 +236,24 @@ struct EpiFloat {
         if (a.amax != nullptr) {
 #pragma unroll
           for (int k = 0; k < 16; ++k) {
-            const float2 f = a.out_dtype == DT_F16 ? unpack2<__half>(p[k]) : unpack2<__nv_bfloat16>(p[k]);
+            const float2 f = a.out_dtype == DT_F32 ? unpack2<E>(p[k])
+                           : a.out_dtype == DT_F16 ? unpack2<__half>(p[k]) : unpack2<__nv_bfloat16>(p[k]);
             stored_max = fmaxf(stored_max, fmaxf(fabsf(f.x), fabsf(f.y)));
           }
         }
-        wp.write_own_row(p);
-        __syncwarp();
-        uint8_t* out = static_cast<uint8_t*>(a.out);
-        if (!a.transpose)
-          store_block_rows(wp, out + ((size_t(t.b) * g.lm + wrow0) * g.ln + colb) * 2, size_t(g.ln) * 2);
-        else
-          store_block_columns16(wp, out + ((size_t(t.b) * g.ln + colb) * g.lm + wrow0) * 2, size_t(g.lm) * 2);
-        __syncwarp();
+        store_final(g, a, t, wp, p, wrow0, colb, EDGE ? BlockClip{g.lm - wrow0, g.ln - colb} : BlockClip{32, 32});
       } else {
         wp.write_own_row(p);
         __syncwarp();
         uint8_t* out = static_cast<uint8_t*>(a.out);
-        store_block_rows(wp, out + ((size_t(t.b) * g.m + wrow0) * g.n + colb) * 2, size_t(g.n) * 2);
-        // transposed copy: the mirrored half of a symmetric product, or the (n x m) transpose
-        // that the next update GEMM consumes (a diagonal tile is bitwise symmetric already)
+        store_block_rows(wp, out + ((size_t(t.b) * g.m + wrow0) * g.n + colb) * 2, size_t(g.n) * 2, held.rows, 2 * held.cols);
+        // transposed copy: the mirrored half of a symmetric product, or an (n x m) transpose that the caller asked
+        // for (a diagonal tile is bitwise symmetric already)
         uint8_t* tdst = mirror ? out : static_cast<uint8_t*>(a.out_t);
         if (tdst != nullptr && !diag_tile) {
           const int tld = mirror ? g.n : g.m;
           store_block_columns16(wp, tdst + ((size_t(t.b) * (mirror ? g.m : g.n) + colb) * tld + wrow0) * 2,
-                                size_t(tld) * 2);
+                                size_t(tld) * 2, held.cols, 2 * held.rows);
         }
         __syncwarp();   // the patch is free for the next chunk
       }
@@ -228,7 +271,8 @@ struct EpiFloat {
                                              const Acc& acc) {
     if constexpr (!IS_F32 && !Acc::IN_REGS) {
       if (fast_ok(g, a, t)) {   // uniform over the tile's warps
-        run_fast(g, a, t, acc);
+        if (t.row0 + TILE > g.lm || t.col0 + TILE > g.ln) run_fast<true>(g, a, t, acc);
+        else run_fast<false>(g, a, t, acc);
         return;
       }
     }

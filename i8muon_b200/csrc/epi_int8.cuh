@@ -48,17 +48,17 @@ struct EpiI8 {
   static constexpr uint32_t IDESC = make_idesc(2u, 1u, 1u, TILE, TILE);  // s32 <- s8 * s8
   using Args = I8Args;
 
-  // Fast path for a tile inside the logical extent: every global access of a warp's 32-row block
-  // goes through the warp's shared-memory patch in coalesced requests, the column diagonal is
-  // loaded once per chunk (one column per lane) and handed round by shuffles.
-  // Every element goes through the same operations, in the same order, as in the general path.
+  // Fast path: every global access of a warp's 32-row block goes through the warp's shared-memory patch in coalesced
+  // requests, clipped to the matrix on its edges; the column diagonal is loaded once per chunk (one column per lane)
+  // and handed round by shuffles.  Padding needs no mask: its operands are zero, so are its results, and a zero
+  // changes no maximum.  Every element goes through the same operations, in the same order, as in the general path.
   static __device__ __forceinline__ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
   static __device__ __forceinline__ bool fast_ok(const GemmGeom& g, const Args& a, const TileCtx& t) {
-    if (t.wsm == nullptr || t.row0 + TILE > g.lm || t.col0 + TILE > g.ln || !aligned16(a.out)) return false;
+    if (t.wsm == nullptr) return false;
     if constexpr (MODE == I8_UPDATE_FINAL) {
-      if (a.out_dtype == DT_F32) { if (a.transpose || (g.ln & 3)) return false; }
-      else if ((a.transpose ? g.lm : g.ln) & 7) return false;
-    } else if (g.n & 3) {
+      if (a.transpose && (a.out_dtype == DT_F32 || !aligned16(a.out) || (g.lm & 7) || t.row0 + TILE > g.lm || t.col0 + TILE > g.ln))
+        return false;
+    } else if (!aligned16(a.out) || (g.n & 3)) {
       return false;
     }
     if constexpr (MODE == I8_SQUARE) return aligned16(g.a_raw) && (g.k & 15) == 0;
@@ -71,7 +71,7 @@ struct EpiI8 {
 
   // 32 columns of 32-bit results per lane row: two halves of 64 bytes through the patch
   static __device__ __forceinline__ void store_rows32(const WarpPatch& wp, uint8_t* dst, size_t pitch,
-                                                      const uint32_t (&r)[32]) {
+                                                      const uint32_t (&r)[32], const BlockClip clip, bool vectors = true) {
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       uint32_t half[16];
@@ -79,12 +79,13 @@ struct EpiI8 {
       for (int k = 0; k < 16; ++k) half[k] = r[16 * h + k];
       wp.write_own_row(half);
       __syncwarp();
-      store_block_rows(wp, dst + 64 * h, pitch);
+      if (vectors) store_block_rows(wp, dst + 64 * h, pitch, clip.rows, 4 * (clip.cols - 16 * h));
+      else store_block_elements32(wp, reinterpret_cast<uint32_t*>(dst + 64 * h), pitch / 4, clip.rows, clip.cols - 16 * h);
       __syncwarp();
     }
   }
 
-  template <class Acc>
+  template <bool EDGE, class Acc>   // EDGE: the tile reaches beyond the logical extents
   static __device__ __forceinline__ void run_fast(const GemmGeom& g, const Args& a, const TileCtx& t,
                                                   const Acc& acc) {
     int imax = 0;
@@ -92,7 +93,7 @@ struct EpiI8 {
     float sa = 0.f, sb = 0.f, sq = 0.f, drow = 0.f, xrow = 0.f;
     if constexpr (MODE != I8_GRAM) {
       sa = a.a_scale[t.b];
-      drow = a.diag[size_t(t.b) * g.m + t.row];
+      if (!EDGE || t.row < g.m) drow = a.diag[size_t(t.b) * g.m + t.row];
     }
     if constexpr (MODE == I8_SQUARE) {
       sq = __fmul_rn(__fmul_rn(sa, sa), a.beta);
@@ -109,26 +110,31 @@ struct EpiI8 {
       uint32_t v[32];
       acc.load(c, v);
       const int colb = t.col0 + c * 32;
+      if (EDGE && (colb >= g.n || wrow0 >= g.m)) continue;       // uniform over the warp
+      // what the padded matrix holds of this block
+      const BlockClip held = EDGE ? BlockClip{g.m - wrow0, g.n - colb} : BlockClip{32, 32};
       const size_t wbase = (size_t(t.b) * g.m + wrow0) * g.n + colb;   // first element of the warp's block
       const int dcol = t.row - colb;   // this row's diagonal column inside the chunk when 0 <= dcol < 32
       if constexpr (MODE == I8_GRAM) {
 #pragma unroll
         for (int j = 0; j < 32; ++j)
           if (j != dcol) imax = max(imax, abs(int(v[j])));
-        store_rows32(wp, reinterpret_cast<uint8_t*>(static_cast<int*>(a.out) + wbase), size_t(g.n) * 4, v);
+        store_rows32(wp, reinterpret_cast<uint8_t*>(static_cast<int*>(a.out) + wbase), size_t(g.n) * 4, v, held);
       } else {
         // the int8 companion block (g8 for the square, a8 for the update): coalesced into the patch
         const int8_t* comp = (MODE == I8_SQUARE)
             ? static_cast<const int8_t*>(g.a_raw) + (size_t(t.b) * g.m + wrow0) * g.k + colb
             : a.row_b + wbase;
-        load_block_rows32(wp, reinterpret_cast<const uint8_t*>(comp), size_t(MODE == I8_SQUARE ? g.k : g.n));
+        load_block_rows32(wp, reinterpret_cast<const uint8_t*>(comp), size_t(MODE == I8_SQUARE ? g.k : g.n),
+                          held.rows, held.cols);
         __syncwarp();
         const uint4 c0 = lds128u(wp.piece(t.lane, 0)), c1 = lds128u(wp.piece(t.lane, 1));
         __syncwarp();
         const uint32_t cw[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
         float cj_lane = 0.f;
         if constexpr (MODE == I8_SQUARE)
-          cj_lane = __fmul_rn(__fmul_rn(a.diag[size_t(t.b) * g.m + colb + t.lane], sa), a.beta);
+          if (!EDGE || colb + t.lane < g.m)
+            cj_lane = __fmul_rn(__fmul_rn(a.diag[size_t(t.b) * g.m + colb + t.lane], sa), a.beta);
         uint32_t res[32];
 #pragma unroll
         for (int j = 0; j < 32; ++j) {
@@ -147,8 +153,10 @@ struct EpiI8 {
         }
         if constexpr (MODE == I8_UPDATE_FINAL) {
           uint8_t* out = static_cast<uint8_t*>(a.out);
+          const BlockClip clip = EDGE ? BlockClip{g.lm - wrow0, g.ln - colb} : BlockClip{32, 32};
           if (a.out_dtype == DT_F32) {
-            store_rows32(wp, out + ((size_t(t.b) * g.lm + wrow0) * g.ln + colb) * 4, size_t(g.ln) * 4, res);
+            store_rows32(wp, out + ((size_t(t.b) * g.lm + wrow0) * g.ln + colb) * 4, size_t(g.ln) * 4, res, clip,
+                         aligned16(a.out) && (g.ln & 3) == 0);
           } else {
             uint32_t p[16];
 #pragma unroll
@@ -158,14 +166,17 @@ struct EpiI8 {
             }
             wp.write_own_row(p);
             __syncwarp();
-            if (!a.transpose)
-              store_block_rows(wp, out + ((size_t(t.b) * g.lm + wrow0) * g.ln + colb) * 2, size_t(g.ln) * 2);
+            const size_t first = (size_t(t.b) * g.lm + wrow0) * g.ln + colb;
+            if (!a.transpose && aligned16(a.out) && (g.ln & 7) == 0)
+              store_block_rows(wp, out + first * 2, size_t(g.ln) * 2, clip.rows, clip.cols * 2);
+            else if (!a.transpose)
+              store_block_elements16(wp, static_cast<uint16_t*>(a.out) + first, size_t(g.ln), clip.rows, clip.cols);
             else
               store_block_columns16(wp, out + ((size_t(t.b) * g.ln + colb) * g.lm + wrow0) * 2, size_t(g.lm) * 2);
             __syncwarp();
           }
         } else {
-          store_rows32(wp, reinterpret_cast<uint8_t*>(static_cast<float*>(a.out) + wbase), size_t(g.n) * 4, res);
+          store_rows32(wp, reinterpret_cast<uint8_t*>(static_cast<float*>(a.out) + wbase), size_t(g.n) * 4, res, held);
         }
       }
     }
@@ -184,7 +195,8 @@ struct EpiI8 {
                                              const Acc& acc) {
     if constexpr (!Acc::IN_REGS) {
       if (fast_ok(g, a, t)) {   // uniform over the tile's warps
-        run_fast(g, a, t, acc);
+        if (t.row0 + TILE > g.lm || t.col0 + TILE > g.ln) run_fast<true>(g, a, t, acc);
+        else run_fast<false>(g, a, t, acc);
         return;
       }
     }

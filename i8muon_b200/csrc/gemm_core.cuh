@@ -3,6 +3,10 @@
 //   A  is (batch, m, k) row-major  -> "K-major" operand tile of 128 rows
 //   Bt is (batch, n, k) row-major  -> rows of B^T, also K-major
 //
+// Either operand may instead be stored with its rows along K - A as (batch, k, m), B as (batch, k, n) - and is
+// then read through the MN-major form of the shared-memory descriptor (geom.a_mn / geom.b_mn).  The matrix that
+// one product reads along K and the next one across it is therefore stored once: no transposed copies.
+//
 // One CTA produces one 128 x 128 output tile.
 //   warp 0      TMA producer: cp.async.bulk.tensor 3-D boxes {128 bytes of K, 128 rows, 1 batch}
 //               with the 128-byte swizzle into a STAGES-deep shared-memory ring
@@ -50,6 +54,8 @@ struct GemmGeom {
   int tiles_per_batch;
   int num_kb;           // K blocks of 128 bytes
   int debug_simt;
+  int a_mn, b_mn;       // operand stored (batch, k, m) / (batch, k, n): MN-major tiles
+  int narrow;           // persistent whole-K kernel: units of one tile instead of two
   int group;            // row blocks per group of the tile / unit order (even, >= 8; set by the launcher)
   const void* a_raw;    // raw operand pointers (debug core and epilogue reads)
   const void* b_raw;
@@ -121,6 +127,53 @@ __host__ __device__ __forceinline__ void decode_tile(const GemmGeom& g, int line
   }
 }
 
+// ------------------------------------------------------- operand tiles
+// A 128-row tile of one 128-byte K block is 16 KB in shared memory either way.
+//   K-major   box {128 bytes of K, 128 rows}: row r of the tile is 128 bytes of K
+//   MN-major  16-bit: two boxes {64 elements, 64 k}, 8-bit: one box {128 elements, 128 k}: a row is 128 bytes
+//             along M / N at one k; eight k rows make a swizzle atom of 1 KB (stride byte offset), the next 64
+//             elements (16-bit) or the next tile (8-bit) are one box away (leading byte offset)
+// The layouts are compile-time constants of the producer's and the issuer's loops (with_layouts picks the
+// instance): with run-time descriptor steps the issuing thread's loop, a serial chain, made FP32 calls 2 % and INT8
+// calls of 768-wide matrices 5 % slower.
+template <typename Elem, int A_MN, int B_MN>
+struct OperandTiles {
+  static constexpr int ES = int(sizeof(Elem));
+  static constexpr int BKE = 128 / ES;                    // elements of one K block
+  static constexpr uint32_t MN_BOX_BYTES = ES == 2 ? TILE_BYTES / 2 : TILE_BYTES;
+  // descriptor advance of one instruction (32 bytes of K), in 16-byte units: inside the swizzle row, or 32 / ES k rows
+  static constexpr uint64_t MN_STEP = 32 / ES * 128 / 16;
+  static constexpr uint64_t A_STEP = A_MN ? MN_STEP : 2, B_STEP = B_MN ? MN_STEP : 2;
+  static constexpr uint32_t IDESC_BITS = (A_MN ? 1u << 15 : 0u) | (B_MN ? 1u << 16 : 0u);   // "transpose" bits
+  template <int MN>
+  static __device__ __forceinline__ void load(uint32_t dst, const CUtensorMap* map, uint32_t bar, int kb, int r0, int b) {
+    if constexpr (!MN) {
+      tma_load_3d(dst, map, bar, kb * BKE, r0, b);
+    } else {
+      tma_load_3d(dst, map, bar, r0, kb * BKE, b);
+      if constexpr (ES == 2) tma_load_3d(dst + MN_BOX_BYTES, map, bar, r0 + 64, kb * BKE, b);
+    }
+  }
+  static __device__ __forceinline__ void load_a(uint32_t dst, const CUtensorMap* map, uint32_t bar, int kb, int r0, int b) {
+    load<A_MN>(dst, map, bar, kb, r0, b);
+  }
+  static __device__ __forceinline__ void load_b(uint32_t dst, const CUtensorMap* map, uint32_t bar, int kb, int r0, int b) {
+    load<B_MN>(dst, map, bar, kb, r0, b);
+  }
+  static __device__ __forceinline__ uint64_t desc_a(uint32_t saddr) { return make_smem_desc_sw128(saddr, A_MN ? MN_BOX_BYTES : 16u); }
+  static __device__ __forceinline__ uint64_t desc_b(uint32_t saddr) { return make_smem_desc_sw128(saddr, B_MN ? MN_BOX_BYTES : 16u); }
+};
+template <typename Elem, class F>
+__device__ __forceinline__ void with_layouts(const GemmGeom& g, F&& f) {
+  if constexpr (sizeof(Elem) == 4) {
+    f(OperandTiles<Elem, 0, 0>{});
+  } else {
+    if (!g.a_mn && !g.b_mn) f(OperandTiles<Elem, 0, 0>{});
+    else if (!g.a_mn) f(OperandTiles<Elem, 0, 1>{});
+    else f(OperandTiles<Elem, 1, 1>{});
+  }
+}
+
 // ----------------------------------------------------- element conversions
 template <int KIND, typename Elem>
 struct ElemOps;
@@ -143,8 +196,11 @@ __device__ __forceinline__ float e4m3_to_float(uint8_t v) {
 template <int KIND, typename Elem>
 __device__ inline uint32_t simt_dot(const GemmGeom& g, int b, int row, int col, int k0, int k1) {
   if (row >= g.m || col >= g.n) return 0u;
-  const Elem* a = static_cast<const Elem*>(g.a_raw) + (size_t(b) * g.m + row) * g.k;
-  const Elem* bt = static_cast<const Elem*>(g.b_raw) + (size_t(b) * g.n + col) * g.k;
+  struct Strided { const Elem* p; size_t step; __device__ Elem operator[](int i) const { return p[size_t(i) * step]; } };
+  const Elem* a0 = static_cast<const Elem*>(g.a_raw) + size_t(b) * g.m * g.k;
+  const Elem* b0 = static_cast<const Elem*>(g.b_raw) + size_t(b) * g.n * g.k;
+  const Strided a{g.a_mn ? a0 + row : a0 + size_t(row) * g.k, g.a_mn ? size_t(g.m) : 1};
+  const Strided bt{g.b_mn ? b0 + col : b0 + size_t(col) * g.k, g.b_mn ? size_t(g.n) : 1};
   if (k1 > g.k) k1 = g.k;
   if constexpr (KIND == KIND_I8) {
     int acc = 0;
@@ -277,6 +333,8 @@ ns_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     // ------------------------------------------------------------ producer
     int issued = 0;
     bool ok = true;
+    with_layouts<typename Epi::Elem>(g, [&](auto tiles) {
+    using Tiles = decltype(tiles);
     for (int kb = 0; kb < g.num_kb; ++kb) {
       const int s = kb % STAGES;
       if (kb >= STAGES) {
@@ -286,14 +344,15 @@ ns_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       const uint32_t bar = smem_u32(&ctrl->full[s]);
       const uint32_t dst = smem_base + uint32_t(s * STAGE_BYTES);
       mbar_arrive_expect_tx(bar, STAGE_BYTES);
-      tma_load_3d(dst, &map_a, bar, kb * BKE, row0, b);
-      tma_load_3d(dst + PARTS * TILE_BYTES, &map_b, bar, kb * BKE, col0, b);
+      Tiles::load_a(dst, &map_a, bar, kb, row0, b);
+      Tiles::load_b(dst + PARTS * TILE_BYTES, &map_b, bar, kb, col0, b);
       if constexpr (PARTS == 2) {
         tma_load_3d(dst + TILE_BYTES, &map_a2, bar, kb * BKE, row0, b);
         tma_load_3d(dst + 3 * TILE_BYTES, &map_b2, bar, kb * BKE, col0, b);
       }
       issued = kb + 1;
     }
+    });
     if (!ok) {
       atomicCAS(g.status, 0u, unsigned(ST_PRODUCER_TIMEOUT) | unsigned(blockIdx.x & 0xff));
       // Let the copies that were issued land before shared memory is released.
@@ -308,13 +367,16 @@ ns_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   } else if (!DEBUG && warp == 1 && lane == 0) {
     // ---------------------------------------------------------- MMA issuer
     bool ok = true;
+    with_layouts<typename Epi::Elem>(g, [&](auto tiles) {
+    using Tiles = decltype(tiles);
     for (int kb = 0; kb < g.num_kb; ++kb) {
       const int s = kb % STAGES;
       ok = mbar_wait(smem_u32(&ctrl->full[s]), uint32_t(kb / STAGES) & 1u, abort_flag);
       if (!ok) break;
       uint32_t d = tmem_base;
-      bool chunk_first = kb == 0, chunk_last = false;
-      int buf = 0;
+      bool chunk_first = kb == 0;
+      [[maybe_unused]] bool chunk_last = false;
+      [[maybe_unused]] int buf = 0;
       if constexpr (PROMOTE > 0) {
         const int chunk = kb / PROMOTE;
         buf = chunk % NBUF;
@@ -332,16 +394,15 @@ ns_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       tc_fence_after();
       const uint32_t sa = smem_base + uint32_t(s * STAGE_BYTES);
       const uint32_t sb = sa + PARTS * TILE_BYTES;
-      const uint64_t adesc = make_smem_desc_sw128(sa);
-      const uint64_t bdesc = make_smem_desc_sw128(sb);
+      const uint64_t adesc = Tiles::desc_a(sa);
+      const uint64_t bdesc = Tiles::desc_b(sb);
 #pragma unroll
       for (int ks = 0; ks < 4; ++ks) {
-        // 32 bytes of K per instruction: advance the start address inside the
-        // 128-byte swizzle row (address field is in 16-byte units).
-        const uint64_t adv = uint64_t(ks * 2);
         uint32_t accumulate = (chunk_first && ks == 0) ? 0u : 1u;
-        umma<Epi::KIND>(d, adesc + adv, bdesc + adv, Epi::IDESC, accumulate);
+        umma<Epi::KIND>(d, adesc + uint64_t(ks) * Tiles::A_STEP, bdesc + uint64_t(ks) * Tiles::B_STEP,
+                        Epi::IDESC | Tiles::IDESC_BITS, accumulate);
         if constexpr (PARTS == 2) {
+          const uint64_t adv = uint64_t(ks * 2);   // both planes K-major
           // split-TF32: hi*hi (above) + hi*lo + lo*hi
           const uint64_t a2 = make_smem_desc_sw128(sa + TILE_BYTES) + adv;
           const uint64_t b2 = make_smem_desc_sw128(sb + TILE_BYTES) + adv;
@@ -357,6 +418,7 @@ ns_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         if (chunk_last) umma_commit(smem_u32(&ctrl->acc_full[buf]));
       }
     }
+    });
     if constexpr (PROMOTE == 0) {
       if (ok) umma_commit(smem_u32(&ctrl->acc_full[0]));
     }
@@ -499,34 +561,73 @@ struct WarpPatch {
   }
 };
 
+// How much of a warp's 32 x 32 block exists: blocks on the edge of a matrix are clipped to its extents, the
+// others are whole.  `rows` and `cols` may be negative (nothing exists).
+struct BlockClip {
+  int rows, cols;
+  __device__ __forceinline__ bool whole() const { return rows >= 32 && cols >= 32; }
+};
+
 // Row-major store of a warp's 32 x 64-byte block held one row per lane: through the patch, as four
-// requests of eight 64-byte row segments.  dst = address of the block's first byte, pitch in bytes.
-__device__ __forceinline__ void store_block_rows(const WarpPatch& wp, uint8_t* dst, size_t pitch) {
+// requests of eight 64-byte row segments.  dst = address of the block's first byte, pitch in bytes; rows and
+// bytes of a row that exist (the latter in whole 16-byte pieces).
+__device__ __forceinline__ void store_block_rows(const WarpPatch& wp, uint8_t* dst, size_t pitch, int rows = 32,
+                                                 int row_bytes = 64) {
 #pragma unroll
   for (int j = 0; j < 4; ++j)
-    *reinterpret_cast<uint4*>(dst + size_t(wp.sweep_row(j)) * pitch + 16 * (wp.lane & 3)) = wp.read_sweep(j);
+    if (wp.sweep_row(j) < rows && 16 * (wp.lane & 3) < row_bytes)
+      *reinterpret_cast<uint4*>(dst + size_t(wp.sweep_row(j)) * pitch + 16 * (wp.lane & 3)) = wp.read_sweep(j);
 }
 // Transposed store of a block of 16-bit values that sits in the patch: column c of the block
 // becomes 64 contiguous bytes at dst + c * pitch.
-__device__ __forceinline__ void store_block_columns16(const WarpPatch& wp, uint8_t* dst, size_t pitch) {
+__device__ __forceinline__ void store_block_columns16(const WarpPatch& wp, uint8_t* dst, size_t pitch, int cols = 32,
+                                                      int col_bytes = 64) {
 #pragma unroll
   for (int i = 0; i < 4; ++i)
-    *reinterpret_cast<uint4*>(dst + size_t(8 * i + (wp.lane >> 2)) * pitch + 16 * (wp.lane & 3)) = wp.read_column(i);
+    if (8 * i + (wp.lane >> 2) < cols && 16 * (wp.lane & 3) < col_bytes)
+      *reinterpret_cast<uint4*>(dst + size_t(8 * i + (wp.lane >> 2)) * pitch + 16 * (wp.lane & 3)) = wp.read_column(i);
+}
+// Row-major store of 16-bit values whose rows start anywhere: one element per lane, a row of up to 32 elements per
+// request.  Matrices with an odd number of columns have no aligned vectors to store.
+__device__ __forceinline__ void store_block_elements16(const WarpPatch& wp, uint16_t* dst, size_t pitch, int rows, int cols) {
+  const uint32_t within = uint32_t((wp.lane & 7) * 2);
+#pragma unroll 8
+  for (int r = 0; r < 32; ++r)
+    if (r < rows && wp.lane < cols) dst[size_t(r) * pitch + wp.lane] = uint16_t(lds16u(wp.piece(r, wp.lane >> 3) + within));
+}
+// The same for 32-bit values: a block of 32 x 16, two rows per request.
+__device__ __forceinline__ void store_block_elements32(const WarpPatch& wp, uint32_t* dst, size_t pitch, int rows, int cols) {
+  const int c = wp.lane & 15;
+  const uint32_t within = uint32_t((c & 3) * 4);
+#pragma unroll 8
+  for (int i = 0; i < 16; ++i) {
+    const int r = 2 * i + (wp.lane >> 4);
+    if (r < rows && c < cols) dst[size_t(r) * pitch + c] = lds32u(wp.piece(r, c >> 2) + within);
+  }
 }
 // Row-major load of a 32 x 32-byte block (int8 companions) into pieces 0 and 1 of the patch rows:
 // two requests of sixteen 32-byte row segments; afterwards lane r finds its row in pieces 0, 1.
-__device__ __forceinline__ void load_block_rows32(const WarpPatch& wp, const uint8_t* src, size_t pitch) {
+__device__ __forceinline__ void load_block_rows32(const WarpPatch& wp, const uint8_t* src, size_t pitch, int rows,
+                                                  int row_bytes) {
 #pragma unroll
   for (int j = 0; j < 2; ++j) {
     const int r = 16 * j + (wp.lane >> 1);
-    sts128u(wp.piece(r, wp.lane & 1), *reinterpret_cast<const uint4*>(src + size_t(r) * pitch + 16 * (wp.lane & 1)));
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    if (r < rows && 16 * (wp.lane & 1) < row_bytes)
+      v = *reinterpret_cast<const uint4*>(src + size_t(r) * pitch + 16 * (wp.lane & 1));
+    sts128u(wp.piece(r, wp.lane & 1), v);
   }
 }
-// Row-major load of a 32 x 64-byte block into the patch (four coalesced requests).
-__device__ __forceinline__ void load_block_rows(const WarpPatch& wp, const uint8_t* src, size_t pitch) {
+// Row-major load of a 32 x 64-byte block into the patch (four coalesced requests); what does not exist reads as zero.
+__device__ __forceinline__ void load_block_rows(const WarpPatch& wp, const uint8_t* src, size_t pitch, int rows = 32,
+                                                int row_bytes = 64) {
 #pragma unroll
-  for (int j = 0; j < 4; ++j)
-    wp.write_sweep(j, *reinterpret_cast<const uint4*>(src + size_t(wp.sweep_row(j)) * pitch + 16 * (wp.lane & 3)));
+  for (int j = 0; j < 4; ++j) {
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    if (wp.sweep_row(j) < rows && 16 * (wp.lane & 3) < row_bytes)
+      v = *reinterpret_cast<const uint4*>(src + size_t(wp.sweep_row(j)) * pitch + 16 * (wp.lane & 3));
+    wp.write_sweep(j, v);
+  }
 }
 
 __device__ __forceinline__ float warp_max(float v) {

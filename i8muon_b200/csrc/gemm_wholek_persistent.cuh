@@ -45,7 +45,6 @@ wholek_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   constexpr int STAGES = WKP_STAGES;
   constexpr int STAGE_BYTES = 2 * TILE_BYTES;
   constexpr int NBUF = WKP_NBUF;
-  constexpr int BKE = 128 / int(sizeof(typename Epi::Elem));  // elements per 128-byte K block
   static_assert(Epi::PARTS == 1 && Epi::PROMOTE_KB == 0 && !Epi::BLOCKQ, "whole-K epilogues only");
   static_assert(STAGES % 2 == 0, "each stream owns half of the stages");
   constexpr int SSTAGES = STAGES / 2;  // stages of one stream: stream, stream + 2, ...
@@ -99,6 +98,8 @@ wholek_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       uint32_t wrap = 0;
       int issued = 0;
       bool ok = true;
+      with_layouts<typename Epi::Elem>(g, [&](auto tiles) {
+      using Tiles = decltype(tiles);
       for (int j = 0; j < stream_tiles && ok; ++j) {
         int b, tm, tn;
         decode_tile(g, int(blockIdx.x) + (2 * j + stream) * int(gridDim.x), b, tm, tn);
@@ -111,12 +112,13 @@ wholek_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
           const uint32_t bar = full0 + 8u * uint32_t(s);
           const uint32_t dst = smem_base + uint32_t(s * STAGE_BYTES);
           mbar_arrive_expect_tx(bar, STAGE_BYTES);
-          tma_load_3d(dst, &map_a, bar, kb * BKE, tm * TILE, b);
-          tma_load_3d(dst + TILE_BYTES, &map_b, bar, kb * BKE, tn * TILE, b);
+          Tiles::load_a(dst, &map_a, bar, kb, tm * TILE, b);
+          Tiles::load_b(dst + TILE_BYTES, &map_b, bar, kb, tn * TILE, b);
           ++issued;
           if (++ring == SSTAGES) { ring = 0; ++wrap; }
         }
       }
+      });
       if (!ok) {
         atomicCAS(g.status, 0u, unsigned(ST_PRODUCER_TIMEOUT) | unsigned(blockIdx.x & 0xff));
         // let the copies that were issued land before shared memory is released
@@ -133,6 +135,8 @@ wholek_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       int ring = 0;
       uint32_t wrap = 0;
       bool ok = true;
+      with_layouts<typename Epi::Elem>(g, [&](auto tiles) {
+      using Tiles = decltype(tiles);
       for (int j = 0; j < stream_tiles && ok; ++j) {
         const int buf = 2 * stream + (j & 1);
         const uint32_t use = uint32_t(j >> 1);  // how often this accumulator was filled before
@@ -147,18 +151,20 @@ wholek_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
           if (!ok) break;
           tc_fence_after();
           const uint32_t sa = smem_base + uint32_t(s * STAGE_BYTES);
-          const uint64_t adesc = make_smem_desc_sw128(sa);
-          const uint64_t bdesc = make_smem_desc_sw128(sa + TILE_BYTES);
+          const uint64_t adesc = Tiles::desc_a(sa);
+          const uint64_t bdesc = Tiles::desc_b(sa + TILE_BYTES);
 #pragma unroll
           for (int ks = 0; ks < 4; ++ks) {
             const uint32_t accumulate = (kb == 0 && ks == 0) ? 0u : 1u;
-            umma<Epi::KIND>(d, adesc + uint64_t(ks * 2), bdesc + uint64_t(ks * 2), Epi::IDESC, accumulate);
+            umma<Epi::KIND>(d, adesc + uint64_t(ks) * Tiles::A_STEP, bdesc + uint64_t(ks) * Tiles::B_STEP,
+                            Epi::IDESC | Tiles::IDESC_BITS, accumulate);
           }
           umma_commit(empty0 + 8u * uint32_t(s));
           if (++ring == SSTAGES) { ring = 0; ++wrap; }
         }
         if (ok) umma_commit(accf0 + 8u * uint32_t(buf));
       }
+      });
       if (!ok) atomicCAS(g.status, 0u, unsigned(ST_MMA_TIMEOUT) | unsigned(blockIdx.x & 0xff));
     }
   } else {

@@ -45,6 +45,11 @@ __host__ __device__ inline int wide_units_per_batch(int tiles_m, int tiles_n, in
 // then columns of R - 2, R - 4, ... units (rows tm >= 2 tw only).
 __host__ __device__ __forceinline__ void decode_unit(const GemmGeom& g, int units_per_batch, int linear, int& b,
                                                      int& tm, int& tn, int& width) {
+  if (g.narrow) {              // units of one tile, in the tile order of the other kernels
+    width = 1;
+    decode_tile(g, linear, b, tm, tn);
+    return;
+  }
   b = linear / units_per_batch;
   int u = linear - b * units_per_batch;
   const int group = g.group;   // even, >= 2
@@ -100,7 +105,6 @@ wholek_wide_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   constexpr int STAGES = WKW_STAGES;
   constexpr int STAGE_BYTES = WKW_STAGE_BYTES;
   constexpr int NBUF = WKW_NBUF;
-  constexpr int BKE = 128 / int(sizeof(typename Epi::Elem));  // elements per 128-byte K block
   static_assert(Epi::PARTS == 1 && Epi::PROMOTE_KB == 0 && !Epi::BLOCKQ, "whole-K epilogues only");
   // the same instruction descriptor with N = 256
   constexpr uint32_t IDESC_WIDE = (Epi::IDESC & ~(0x3Fu << 17)) | (uint32_t(WKW_ACC_COLS >> 3) << 17);
@@ -139,7 +143,7 @@ wholek_wide_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   const uint32_t full0 = smem_u32(&ctrl->full[0]), empty0 = smem_u32(&ctrl->empty[0]);
   const uint32_t accf0 = smem_u32(&ctrl->acc_full[0]), acce0 = smem_u32(&ctrl->acc_empty[0]);
 
-  const int upb = wide_units_per_batch(g.tiles_m, g.tiles_n, g.sym);
+  const int upb = g.narrow ? g.tiles_per_batch : wide_units_per_batch(g.tiles_m, g.tiles_n, g.sym);
   const int total_units = upb * g.batch;
   const int my_units = (total_units - int(blockIdx.x) + int(gridDim.x) - 1) / int(gridDim.x);
   const int nkb = g.num_kb;
@@ -154,6 +158,8 @@ wholek_wide_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       bool ok = true;
       // test hook (i8m_set_debug_core(2)): issue nothing, so that every consumer's bounded wait runs out
       const int units = (g.debug_simt & 0x100) ? 0 : my_units;
+      with_layouts<typename Epi::Elem>(g, [&](auto tiles) {
+      using Tiles = decltype(tiles);
       for (int j = 0; j < units && ok; ++j) {
         int b, tm, tn, width;
         decode_unit(g, upb, int(blockIdx.x) + j * int(gridDim.x), b, tm, tn, width);
@@ -166,13 +172,14 @@ wholek_wide_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
           const uint32_t bar = full0 + 8u * uint32_t(ring);
           const uint32_t dst = smem_base + uint32_t(ring * STAGE_BYTES);
           mbar_arrive_expect_tx(bar, bytes);
-          tma_load_3d(dst, &map_a, bar, kb * BKE, tm * TILE, b);
-          tma_load_3d(dst + TILE_BYTES, &map_b, bar, kb * BKE, tn * TILE, b);
-          if (width == 2) tma_load_3d(dst + 2 * TILE_BYTES, &map_b, bar, kb * BKE, (tn + 1) * TILE, b);
+          Tiles::load_a(dst, &map_a, bar, kb, tm * TILE, b);
+          Tiles::load_b(dst + TILE_BYTES, &map_b, bar, kb, tn * TILE, b);
+          if (width == 2) Tiles::load_b(dst + 2 * TILE_BYTES, &map_b, bar, kb, (tn + 1) * TILE, b);
           ++issued;
           if (++ring == STAGES) { ring = 0; ++wrap; }
         }
       }
+      });
       if (!ok) {
         atomicCAS(g.status, 0u, unsigned(ST_PRODUCER_TIMEOUT) | unsigned(blockIdx.x & 0xff));
         // let the copies that were issued land before shared memory is released
@@ -189,10 +196,12 @@ wholek_wide_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       int ring = 0;
       uint32_t wrap = 0;
       bool ok = true;
+      with_layouts<typename Epi::Elem>(g, [&](auto tiles) {
+      using Tiles = decltype(tiles);
       for (int j = 0; j < my_units && ok; ++j) {
         int b, tm, tn, width;
         decode_unit(g, upb, int(blockIdx.x) + j * int(gridDim.x), b, tm, tn, width);
-        const uint32_t idesc = width == 2 ? IDESC_WIDE : Epi::IDESC;
+        const uint32_t idesc = (width == 2 ? IDESC_WIDE : Epi::IDESC) | Tiles::IDESC_BITS;
         const int buf = j & 1;
         const uint32_t use = uint32_t(j >> 1);  // how often this accumulator was filled before
         if (use >= 1) {
@@ -205,18 +214,19 @@ wholek_wide_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
           if (!ok) break;
           tc_fence_after();
           const uint32_t sa = smem_base + uint32_t(ring * STAGE_BYTES);
-          const uint64_t adesc = make_smem_desc_sw128(sa);
-          const uint64_t bdesc = make_smem_desc_sw128(sa + TILE_BYTES);   // 128 or 256 rows, 8-row groups 1 KB apart
+          const uint64_t adesc = Tiles::desc_a(sa);
+          const uint64_t bdesc = Tiles::desc_b(sa + TILE_BYTES);   // 128 or 256 rows
 #pragma unroll
           for (int ks = 0; ks < 4; ++ks) {
             const uint32_t accumulate = (kb == 0 && ks == 0) ? 0u : 1u;
-            umma<Epi::KIND>(d, adesc + uint64_t(ks * 2), bdesc + uint64_t(ks * 2), idesc, accumulate);
+            umma<Epi::KIND>(d, adesc + uint64_t(ks) * Tiles::A_STEP, bdesc + uint64_t(ks) * Tiles::B_STEP, idesc, accumulate);
           }
           umma_commit(empty0 + 8u * uint32_t(ring));
           if (++ring == STAGES) { ring = 0; ++wrap; }
         }
         if (ok) umma_commit(accf0 + 8u * uint32_t(buf));
       }
+      });
       if (!ok) atomicCAS(g.status, 0u, unsigned(ST_MMA_TIMEOUT) | unsigned(blockIdx.x & 0xff));
     }
   } else {

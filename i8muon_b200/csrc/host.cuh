@@ -17,7 +17,6 @@ namespace i8m {
 extern thread_local char g_error[512];
 extern thread_local int g_debug_simt;
 extern thread_local int g_starve_producers;   // test hook: see bq_produce
-extern thread_local float* g_final_amax;      // set by run_float around its final product: [batch] maximum of the stored result
 extern thread_local int g_wholek_variant;     // "wholek_gemm": 0 units of 128 x 256, 1 two streams of 128 x 128 tiles, 2 one CTA per tile
 extern thread_local int g_cta_limit;          // persistent GEMM kernels launch at most this many CTAs (0: one per SM)
 // block-quantised GEMMs: 0 = split kernel (tail on its own warps, four-stage ring), 1 = fused tail with a
@@ -73,9 +72,9 @@ inline int cdiv(long long a, long long b) { return int((a + b - 1) / b); }
 inline int pad_to(int v, int a) { return (v + a - 1) / a * a; }
 inline size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
 
-// 3-D map {k, rows, batch} over a (batch, rows, k) row-major operand; the box is {128 bytes of K, 128 rows, 1};
-// rows or K beyond the tensor read as zero.
-int make_operand_map(CUtensorMap* map, const void* ptr, int esize, int k, int rows, int batch);
+// 3-D map over a row-major operand.  K-major: (batch, extent, k), box {128 bytes of K, 128 rows, 1}; MN-major:
+// (batch, k, extent), box {128 bytes along the extent, one K block of rows, 1}.  What lies beyond the tensor reads as zero.
+int make_operand_map(CUtensorMap* map, const void* ptr, int esize, int k, int extent, int batch, int mn = 0);
 int sm_count();   // of the current device, capped by i8m_set_cta_limit
 
 inline bool float_dtype_ok(int d) { return d == I8M_F32 || d == I8M_F16 || d == I8M_BF16; }

@@ -16,34 +16,55 @@ inline int wide_group(long long k_bytes) {
   return int(std::min<long long>(64, std::max<long long>(8, fit))) & ~1;
 }
 
+// Whether the persistent whole-K kernel takes units of one tile (128 x 128) instead of two (128 x 256).  A K block costs
+// about 540 cycles in a pair and 390 alone (both bound by what the SM takes in from L2: 48 and 32 KB at 89 bytes per
+// cycle), a tile's epilogue about 2000, of which only the last one per CTA is not under another unit's K loop.  Pairs
+// win when there are many; with few tiles the number of waves decides.
+inline bool narrow_units(long long tiles, long long pairs, int k_blocks, int ctas) {
+  const long long one = (tiles + ctas - 1) / ctas * k_blocks * 390 + 2000;
+  const long long two = (pairs + ctas - 1) / ctas * k_blocks * 540 + 4000;
+  return one < two;
+}
+
+// One product: operands, extents and what the kernels need besides the epilogue's own arguments.
+struct GemmCall {
+  const void *a = nullptr, *a_lo = nullptr, *b = nullptr, *b_lo = nullptr;   // low planes: FP32 as two TF32 planes
+  int a_mn = 0, b_mn = 0;       // operand stored with its rows along K (GemmGeom)
+  int batch = 0, m = 0, n = 0, k = 0, lm = 0, ln = 0, sym = 0;
+  unsigned* status = nullptr;
+  cudaStream_t stream = nullptr;
+};
+
 template <class Epi>
-int launch_gemm(const void* a, const void* a_lo, const void* bt, const void* bt_lo, int batch,
-                int m, int n, int k, int lm, int ln, int sym, unsigned* status,
-                const typename Epi::Args& args, cudaStream_t stream, const char* name) {
+int launch_gemm(const GemmCall& c, const typename Epi::Args& args, const char* name) {
+  const int batch = c.batch, m = c.m, n = c.n, k = c.k, sym = c.sym;
+  const cudaStream_t stream = c.stream;
   if (batch < 1 || m < 1 || n < 1 || k < 1) return fail(I8M_E_ARGUMENT, "%s: empty problem", name);
-  if (!a || !bt || !status) return fail(I8M_E_ARGUMENT, "%s: null operand or status pointer", name);
+  if (!c.a || !c.b || !c.status) return fail(I8M_E_ARGUMENT, "%s: null operand or status pointer", name);
   if (sym && m != n) return fail(I8M_E_ARGUMENT, "%s: symmetric product needs m == n", name);
   constexpr int ES = int(sizeof(typename Epi::Elem));
   constexpr int STAGE_BYTES = 2 * Epi::PARTS * TILE_BYTES;
   constexpr size_t SMEM = size_t(Epi::STAGES) * STAGE_BYTES + sizeof(Ctrl) + 1024;
-  GemmGeom g;
-  g.batch = batch; g.m = m; g.n = n; g.k = k; g.lm = lm; g.ln = ln;
+  GemmGeom g{};
+  g.batch = batch; g.m = m; g.n = n; g.k = k; g.lm = c.lm; g.ln = c.ln;
   g.tiles_m = cdiv(m, TILE); g.tiles_n = cdiv(n, TILE);
   g.sym = sym;
+  g.a_mn = c.a_mn; g.b_mn = c.b_mn;
   g.tiles_per_batch = sym ? g.tiles_m * (g.tiles_m + 1) / 2 : g.tiles_m * g.tiles_n;
   g.num_kb = cdiv((long long)k * ES, 128);
   g.debug_simt = g_debug_simt | (g_starve_producers ? 0x100 : 0);
   g.group = wide_group((long long)k * ES);
-  g.a_raw = a; g.b_raw = bt; g.status = status;
+  g.a_raw = c.a; g.b_raw = c.b; g.status = c.status;
   long long blocks = (long long)g.tiles_per_batch * batch;
   if (blocks > 0x7fffffffLL) return fail(I8M_E_LIMIT, "%s: too many tiles", name);
   CUtensorMap ma, mb, ma2, mb2;
-  if (int rc = make_operand_map(&ma, a, ES, k, m, batch)) return rc;
-  if (int rc = make_operand_map(&mb, bt, ES, k, n, batch)) return rc;
+  if (int rc = make_operand_map(&ma, c.a, ES, k, m, batch, c.a_mn)) return rc;
+  if (int rc = make_operand_map(&mb, c.b, ES, k, n, batch, c.b_mn)) return rc;
   if (Epi::PARTS == 2) {
-    if (!a_lo || !bt_lo) return fail(I8M_E_ARGUMENT, "%s: missing low planes", name);
-    if (int rc = make_operand_map(&ma2, a_lo, ES, k, m, batch)) return rc;
-    if (int rc = make_operand_map(&mb2, bt_lo, ES, k, n, batch)) return rc;
+    if (!c.a_lo || !c.b_lo) return fail(I8M_E_ARGUMENT, "%s: missing low planes", name);
+    if (c.a_mn || c.b_mn) return fail(I8M_E_ARGUMENT, "%s: two-plane operands are read along K only", name);
+    if (int rc = make_operand_map(&ma2, c.a_lo, ES, k, m, batch)) return rc;
+    if (int rc = make_operand_map(&mb2, c.b_lo, ES, k, n, batch)) return rc;
   } else {
     ma2 = ma; mb2 = mb;
   }
@@ -54,7 +75,9 @@ int launch_gemm(const void* a, const void* a_lo, const void* bt, const void* bt_
       auto wk = wholek_wide_kernel<Epi>;
       static SmemAllowed allowed;
       if (int rc = allow_smem(allowed, wk, WSMEM)) return rc;
-      const long long units = (long long)wide_units_per_batch(g.tiles_m, g.tiles_n, sym) * batch;
+      const long long pairs = (long long)wide_units_per_batch(g.tiles_m, g.tiles_n, sym) * batch;
+      g.narrow = narrow_units(blocks, pairs, g.num_kb, sm_count());
+      const long long units = g.narrow ? blocks : pairs;
       launch(wk, unsigned(std::min<long long>(units, sm_count())), WKW_THREADS, WSMEM, stream, ma, mb, g, args);
       LAUNCH_CHECK(name);
       return 0;
@@ -86,12 +109,16 @@ int launch_gemm(const void* a, const void* a_lo, const void* bt, const void* bt_
 template <class Epi>
 int launch_bq(const void* a, const void* bt, int batch, int m, int n, int k, int lm, int ln, int sym,
               unsigned* status, const typename Epi::Args& args, cudaStream_t stream, const char* name) {
-  if (g_debug_simt)
-    return launch_gemm<Epi>(a, nullptr, bt, nullptr, batch, m, n, k, lm, ln, sym, status, args, stream, name);
+  if (g_debug_simt) {
+    GemmCall c;
+    c.a = a; c.b = bt; c.batch = batch; c.m = m; c.n = n; c.k = k; c.lm = lm; c.ln = ln; c.sym = sym;
+    c.status = status; c.stream = stream;
+    return launch_gemm<Epi>(c, args, name);
+  }
   if (batch < 1 || m < 1 || n < 1 || k < 1) return fail(I8M_E_ARGUMENT, "%s: empty problem", name);
   if (!a || !bt || !status) return fail(I8M_E_ARGUMENT, "%s: null operand or status pointer", name);
   if (sym && m != n) return fail(I8M_E_ARGUMENT, "%s: symmetric product needs m == n", name);
-  GemmGeom g;
+  GemmGeom g{};
   g.batch = batch; g.m = m; g.n = n; g.k = k; g.lm = lm; g.ln = ln;
   g.tiles_m = cdiv(m, TILE); g.tiles_n = cdiv(n, TILE);
   g.sym = sym;

@@ -15,7 +15,6 @@ namespace i8m {
 thread_local char g_error[512] = "";
 thread_local int g_debug_simt = 0;
 thread_local int g_starve_producers = 0;
-thread_local float* g_final_amax = nullptr;
 thread_local int g_wholek_variant = 0;
 thread_local int g_cta_limit = 0;
 thread_local int g_bq_variant = 0;
@@ -63,18 +62,19 @@ int load_encode() {
 }
 }  // namespace
 
-int make_operand_map(CUtensorMap* map, const void* ptr, int esize, int k, int rows, int batch) {
+int make_operand_map(CUtensorMap* map, const void* ptr, int esize, int k, int extent, int batch, int mn) {
+  const int inner = mn ? extent : k, rows = mn ? k : extent;
   if (int rc = load_encode()) return rc;
   if ((reinterpret_cast<uintptr_t>(ptr) & 15u) != 0)
     return fail(I8M_E_ARGUMENT, "GEMM operand is not 16-byte aligned");
-  if ((size_t(k) * esize) % 16 != 0)
-    return fail(I8M_E_ARGUMENT, "GEMM operand row pitch (%d x %d bytes) is not a multiple of 16", k, esize);
+  if ((size_t(inner) * esize) % 16 != 0)
+    return fail(I8M_E_ARGUMENT, "GEMM operand row pitch (%d x %d bytes) is not a multiple of 16", inner, esize);
   CUtensorMapDataType dt = esize == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8
                          : esize == 2 ? CU_TENSOR_MAP_DATA_TYPE_UINT16
                                       : CU_TENSOR_MAP_DATA_TYPE_UINT32;
-  cuuint64_t dims[3] = {cuuint64_t(k), cuuint64_t(rows), cuuint64_t(batch)};
-  cuuint64_t strides[2] = {cuuint64_t(k) * esize, cuuint64_t(k) * esize * rows};
-  cuuint32_t box[3] = {cuuint32_t(128 / esize), 128u, 1u};
+  cuuint64_t dims[3] = {cuuint64_t(inner), cuuint64_t(rows), cuuint64_t(batch)};
+  cuuint64_t strides[2] = {cuuint64_t(inner) * esize, cuuint64_t(inner) * esize * rows};
+  cuuint32_t box[3] = {cuuint32_t(128 / esize), cuuint32_t(mn ? 128 / esize : 128), 1u};
   cuuint32_t estr[3] = {1u, 1u, 1u};
   CUresult r = g_encode(map, dt, 3, const_cast<void*>(ptr), dims, strides, box, estr,
                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
@@ -182,7 +182,15 @@ FMat take_fmat(Bump& ws, size_t elems, int compute) {
   return m;
 }
 
-// floating NS (regular and Gram); with plan == true only the workspace is sized.
+// Restart string of a Gram-space call, padded to the number of iterations.
+int restart_order(const NsCall& c, int steps, std::string& order) {
+  order = c.gram_order ? c.gram_order : "00100";
+  if (order.empty() || order[0] != '0' || order.find_first_not_of("01") != std::string::npos)
+    return fail(I8M_E_ARGUMENT, "gram_order must be a binary string starting with 0");
+  if (int(order.size()) < steps) order.append(size_t(steps) - order.size(), '0');
+  return 0;
+}
+
 struct BqOperands {   // where a floating first row leaves its result for the block-quantised rows
   uint8_t* a = nullptr;
   uint8_t* at = nullptr;
@@ -190,9 +198,110 @@ struct BqOperands {   // where a floating first row leaves its result for the bl
   int lp = 0, hp = 0;
 };
 
-int run_float(const NsCall& c, Bump& ws, bool plan, bool gram, const void* x, void* out,
-              int out_dtype, int steps, const double* coeffs, int compute, bool normalize_input,
-              bool factored = false, const BqOperands* to_bq = nullptr, float* final_amax = nullptr) {
+// Floating NS (regular and Gram) in a 16-bit compute type; with plan == true only the workspace is sized.
+// The matrix X stays in the caller's orientation, padded to multiples of 16, and is stored once: the products that
+// run along its rows read it K-major, those that run across them MN-major.
+//   wide (l x h)   Gram X X^T: both K-major;           update Q X: X is the right operand, MN-major
+//   tall (h x l)   Gram X^T X: both operands MN-major; update X Q: X is the left operand, K-major (Q is symmetric)
+int run_float16(const NsCall& c, Bump& ws, bool plan, bool gram, const void* x, void* out, int out_dtype, int steps,
+                const double* coeffs, int compute, bool normalize_input, bool factored, const BqOperands* to_bq,
+                float* final_amax) {
+  const int B = c.batch, rows = c.rows, cols = c.cols;
+  const int l = std::min(rows, cols), h = std::max(rows, cols);
+  const int lp = pad_to(l, 16), hp = pad_to(h, 16), rp = pad_to(rows, 16), cp = pad_to(cols, 16);
+  const int tall = rows > cols;
+  const size_t es = 2, full = size_t(B) * rp * cp * es, sq = size_t(B) * lp * lp * es;
+  void *a = ws.take(full), *y = ws.take(full);
+  void *r = ws.take(sq), *q0 = ws.take(sq), *z = nullptr, *q1 = nullptr;
+  if (gram) { z = ws.take(sq); q1 = ws.take(sq); }
+  float* norm = ws.take_n<float>(B);
+  const size_t sbytes = stats_bytes(B, (long long)rows * cols);
+  void* scratch = ws.take(sbytes);
+  if (plan) return 0;
+
+  if (normalize_input)
+    if (int rc = call_stats(c, x, B, (long long)rows * cols, scratch, sbytes, norm, nullptr)) return rc;
+  if (int rc = i8m_normalize(x, c.dtype, normalize_input ? norm : nullptr, a, nullptr, nullptr, nullptr, compute, B, rows,
+                             cols, rp, cp, 0, c.eps, c.stream))
+    return rc;
+  FloatGemm base{};
+  base.compute = compute; base.batch = B; base.status = c.status; base.stream = c.stream; base.out_dtype = out_dtype;
+  auto square = [&](const void* left, const void* right, void* o, int mode, double ca, double cb, double cc) {
+    FloatGemm g = base;   // symmetric l x l product of two l x l matrices
+    g.left = left; g.right = right; g.out = o; g.mode = mode;
+    g.m = g.n = g.k = lp; g.lm = g.ln = l; g.symmetric = 1;
+    g.ca = float(ca); g.cb = float(cb); g.cc = float(cc);
+    return float_gemm(g);
+  };
+  auto outer = [&](void* o) {
+    FloatGemm g = base;   // R = X X^T or X^T X
+    g.left = g.right = a; g.left_mn = g.right_mn = tall; g.out = o;
+    g.m = g.n = lp; g.k = hp; g.lm = g.ln = l; g.symmetric = 1;
+    return float_gemm(g);
+  };
+  auto update = [&](const void* q, void* o, int final) {
+    FloatGemm g = base;
+    g.left = tall ? a : q; g.right = tall ? q : a; g.right_mn = !tall;
+    g.out = o; g.final = final; g.amax = final ? final_amax : nullptr;
+    g.m = rp; g.n = cp; g.k = lp; g.lm = rows; g.ln = cols;
+    return float_gemm(g);
+  };
+  if (!gram) {
+    for (int it = 0; it < steps; ++it) {
+      double ca = coeffs[3 * it], cb = coeffs[3 * it + 1], cc = coeffs[3 * it + 2];
+      if (int rc = outer(r)) return rc;
+      if (factored) {
+        // completed-square row (c, p, q): shift the Gram diagonal by p, then c*q I + c R'^2
+        // (src/i8muon/_cutlass_prec.py:97-100)
+        const double fc = ca, fp = cb, fq = cc;
+        if (int rc = add_diagonal(r, compute, B, lp, l, float(fp), c.stream)) return rc;
+        ca = fc * fq; cb = 0.0; cc = fc;
+      }
+      if (int rc = square(r, r, q0, 1, ca, cb, cc)) return rc;
+      const bool final = it == steps - 1;
+      if (final && to_bq)   // the result leaves as INT8 blocks of the wide orientation
+        return float_gemm_to_bq(q0, a, !tall, to_bq->a, to_bq->at, to_bq->sa, compute, out_dtype, B, lp, hp, lp, l, h,
+                                to_bq->lp, to_bq->hp, c.status, c.stream);
+      if (int rc = update(q0, final ? out : y, final)) return rc;
+      std::swap(a, y);
+    }
+    return 0;
+  }
+  // Gram-space iteration with restarts (src/i8muon/_cutlass_prec.py:107-130).
+  std::string order;
+  if (int rc = restart_order(c, steps, order)) return rc;
+  for (int it = 0; it < steps; ++it) {
+    const double ca = coeffs[3 * it], cb = coeffs[3 * it + 1], cc = coeffs[3 * it + 2];
+    const char kind = order[size_t(it)];
+    const bool refresh = it + 1 < steps && order[size_t(it) + 1] == '0';
+    if (kind == '1') {
+      if (int rc = update(q0, y, 0)) return rc;
+      std::swap(a, y);
+    }
+    if (kind == '1' || it == 0) {
+      if (int rc = outer(r)) return rc;
+      if (int rc = square(r, r, q0, 1, ca, cb, cc)) return rc;
+      if (refresh) {
+        if (int rc = square(r, q0, q1, 0, 0, 0, 0)) return rc;
+        if (int rc = square(q0, q1, r, 0, 0, 0, 0)) return rc;
+      }
+    } else {
+      if (int rc = square(r, r, z, 1, ca, cb, cc)) return rc;
+      if (int rc = square(z, q0, q1, 0, 0, 0, 0)) return rc;
+      std::swap(q0, q1);
+      if (refresh) {
+        if (int rc = square(r, z, q1, 0, 0, 0, 0)) return rc;
+        if (int rc = square(z, q1, r, 0, 0, 0, 0)) return rc;
+      }
+    }
+  }
+  return update(q0, out, 1);
+}
+
+// FP32 compute: every matrix as two planes, X and its transpose both stored (TF32 operands are read K-major only).
+int run_float32(const NsCall& c, Bump& ws, bool plan, bool gram, const void* x, void* out, int out_dtype, int steps,
+                const double* coeffs) {
+  const int compute = I8M_F32;
   const int B = c.batch, rows = c.rows, cols = c.cols;
   const int l = std::min(rows, cols), h = std::max(rows, cols);
   const int lp = pad_to(l, 16), hp = pad_to(h, 16);
@@ -208,19 +317,13 @@ int run_float(const NsCall& c, Bump& ws, bool plan, bool gram, const void* x, vo
   void* scratch = ws.take(sbytes);
   if (plan) return 0;
 
-  if (normalize_input) {
-    if (int rc = call_stats(c, x, B, (long long)rows * cols, scratch, sbytes, norm, nullptr)) return rc;
-  }
-  if (int rc = i8m_normalize(x, c.dtype, normalize_input ? norm : nullptr, a.p, at.p, a.lo, at.lo,
+  if (int rc = call_stats(c, x, B, (long long)rows * cols, scratch, sbytes, norm, nullptr)) return rc;
+  if (int rc = i8m_normalize(x, c.dtype, norm, a.p, at.p, a.lo, at.lo,
                              compute, B, rows, cols, lp, hp, transpose, c.eps, c.stream))
     return rc;
   auto gemm = [&](const FMat& left, const FMat& right, const FMat& o, const FMat& ot, int mode, int n,
                   int k, int ln, int sym, int final, int tr, void* user, double ca, double cb,
                   double cc) -> int {
-    // the final product can leave the maximum magnitude of what it stores (the global-INT8 rows that
-    // follow an FP16 first row quantise it with that scale: no statistics pass over the result)
-    struct Handover { ~Handover() { g_final_amax = nullptr; } } reset;
-    g_final_amax = final ? final_amax : nullptr;
     return i8m_float_gemm(left.p, left.lo, right.p, right.lo, final ? user : o.p, ot.p, o.lo, ot.lo,
                           compute, mode, B, lp, n, k, l, ln, sym, final, tr, out_dtype, float(ca),
                           float(cb), float(cc), c.status, c.stream);
@@ -228,34 +331,18 @@ int run_float(const NsCall& c, Bump& ws, bool plan, bool gram, const void* x, vo
   const FMat none;
   if (!gram) {
     for (int it = 0; it < steps; ++it) {
-      double ca = coeffs[3 * it], cb = coeffs[3 * it + 1], cc = coeffs[3 * it + 2];
+      const double ca = coeffs[3 * it], cb = coeffs[3 * it + 1], cc = coeffs[3 * it + 2];
       if (int rc = gemm(a, a, r, none, 0, lp, hp, l, 1, 0, 0, nullptr, 0, 0, 0)) return rc;
-      if (factored) {
-        // completed-square row (c, p, q): shift the Gram diagonal by p, then c*q I + c R'^2
-        // (src/i8muon/_cutlass_prec.py:97-100); 16-bit compute types only
-        const double fc = ca, fp = cb, fq = cc;
-        if (int rc = add_diagonal(r.p, compute, B, lp, l, float(fp), c.stream)) return rc;
-        ca = fc * fq; cb = 0.0; cc = fc;
-      }
       if (int rc = gemm(r, r, q0, none, 1, lp, lp, l, 1, 0, 0, nullptr, ca, cb, cc)) return rc;
       const bool final = it == steps - 1;
-      if (final && to_bq) {
-        // the result stays in the wide orientation and leaves as INT8 blocks (no transposition back)
-        if (int rc = i8m_float_gemm_to_bq(q0.p, at.p, to_bq->a, to_bq->at, to_bq->sa, compute, out_dtype, B, lp, hp, lp,
-                                          l, h, to_bq->lp, to_bq->hp, c.status, c.stream))
-          return rc;
-        return 0;
-      }
       if (int rc = gemm(q0, at, y, yt, 0, hp, lp, h, 0, final, final && transpose, out, 0, 0, 0)) return rc;
       if (!final) { std::swap(a, y); std::swap(at, yt); }
     }
     return 0;
   }
   // Gram-space iteration with restarts (src/i8muon/_cutlass_prec.py:107-130).
-  std::string order = c.gram_order ? c.gram_order : "00100";
-  if (order.empty() || order[0] != '0' || order.find_first_not_of("01") != std::string::npos)
-    return fail(I8M_E_ARGUMENT, "gram_order must be a binary string starting with 0");
-  if (int(order.size()) < steps) order.append(size_t(steps) - order.size(), '0');
+  std::string order;
+  if (int rc = restart_order(c, steps, order)) return rc;
   for (int it = 0; it < steps; ++it) {
     const double ca = coeffs[3 * it], cb = coeffs[3 * it + 1], cc = coeffs[3 * it + 2];
     const char kind = order[size_t(it)];
@@ -282,6 +369,13 @@ int run_float(const NsCall& c, Bump& ws, bool plan, bool gram, const void* x, vo
     }
   }
   return gemm(q0, at, y, yt, 0, hp, lp, h, 0, 1, transpose, out, 0, 0, 0);
+}
+
+int run_float(const NsCall& c, Bump& ws, bool plan, bool gram, const void* x, void* out, int out_dtype, int steps,
+              const double* coeffs, int compute, bool normalize_input, bool factored = false,
+              const BqOperands* to_bq = nullptr, float* final_amax = nullptr) {
+  if (compute == I8M_F32) return run_float32(c, ws, plan, gram, x, out, out_dtype, steps, coeffs);
+  return run_float16(c, ws, plan, gram, x, out, out_dtype, steps, coeffs, compute, normalize_input, factored, to_bq, final_amax);
 }
 
 // global-scale INT8 NS (src/i8muon/_cutlass.py:162-251)

@@ -60,6 +60,48 @@ __device__ __forceinline__ float block_max_256(float v, float* sh) {
 // elements 8 (t + 256 i) + e of the chunk, i = 0..3 outer, e = 0..7 inner, s = fma(v, v, s) in that order,
 // then the block tree.  Same mapping => bit-identical norms whichever kernel produced the partials.
 template <typename In>
+__device__ __forceinline__ void unpack8(const uint4 raw, float (&v)[8]) {
+  const In* e = reinterpret_cast<const In*>(&raw);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) v[j] = widen<In>(e[j]);
+}
+// eight consecutive input elements (16-byte aligned): one vector load for 16-bit types, two for FP32
+template <typename In>
+__device__ __forceinline__ void load8(const In* p, float (&v)[8]) {
+  if constexpr (sizeof(In) == 4) {
+    const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+  } else {
+    unpack8<In>(*reinterpret_cast<const uint4*>(p), v);
+  }
+}
+
+// This thread's 32 elements of a chunk: four groups of eight, loaded as vectors when x allows it (all four groups in
+// flight before the first is used; with single-element loads 226 MB of BF16 took 62.7 us).
+template <typename In>
+__device__ __forceinline__ void chunk_stats(const In* src, long long base, long long count, float& s, float& mx) {
+  const bool vectors = (reinterpret_cast<uintptr_t>(src) & 15u) == 0 && base + STATS_CHUNK <= count;
+  float v[4][8];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const long long e0 = base + 8 * (threadIdx.x + STATS_THREADS * i);
+    if (vectors) {
+      load8<In>(src + e0, v[i]);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[i][e] = e0 + e < count ? load_f(src, size_t(e0 + e)) : 0.f;
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      s = __fmaf_rn(v[i][e], v[i][e], s);
+      mx = fmaxf(mx, fabsf(v[i][e]));
+    }
+}
+
+template <typename In>
 __global__ void __launch_bounds__(STATS_THREADS)
 stats_partial_kernel(const In* x, float* partial_sum, float* partial_max, long long count,
                      int chunks) {
@@ -69,16 +111,7 @@ stats_partial_kernel(const In* x, float* partial_sum, float* partial_max, long l
   const In* src = x + size_t(b) * count;
   const long long base = (long long)chunk * STATS_CHUNK;
   float s = 0.f, mx = 0.f;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const long long idx = base + 8 * (threadIdx.x + STATS_THREADS * i) + e;
-      const float v = idx < count ? load_f(src, size_t(idx)) : 0.f;
-      s = __fmaf_rn(v, v, s);
-      mx = fmaxf(mx, fabsf(v));
-    }
-  }
+  chunk_stats(src, base, count, s, mx);
   s = block_sum_256(s, sh);
   mx = block_max_256(mx, sh);
   if (threadIdx.x == 0) {
@@ -121,16 +154,7 @@ stats_onepass_kernel(const In* x, float* sumsq, unsigned* amax_bits, unsigned* a
   const In* src = x + size_t(b) * count;
   long long base = (long long)chunk * STATS_CHUNK;
   float s = 0.f, mx = 0.f;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const long long idx = base + 8 * (threadIdx.x + STATS_THREADS * i) + e;
-      const float v = idx < count ? load_f(src, size_t(idx)) : 0.f;
-      s = __fmaf_rn(v, v, s);
-      mx = fmaxf(mx, fabsf(v));
-    }
-  }
+  chunk_stats(src, base, count, s, mx);
   s = block_sum_256(s, sh);
   mx = block_max_256(mx, sh);
   if (threadIdx.x == 0) {
@@ -210,23 +234,6 @@ normalize_kernel(const In* x, const float* norm, E* out, E* out_t, float* out_lo
 // results as the scalar kernels above.
 __device__ __forceinline__ uint32_t swz16(int c) { return uint32_t((c >> 3) & 7) << 4; }
 
-template <typename In>
-__device__ __forceinline__ void unpack8(const uint4 raw, float (&v)[8]) {
-  const In* e = reinterpret_cast<const In*>(&raw);
-#pragma unroll
-  for (int j = 0; j < 8; ++j) v[j] = widen<In>(e[j]);
-}
-// eight consecutive input elements (16-byte aligned): one vector load for 16-bit types, two for FP32
-template <typename In>
-__device__ __forceinline__ void load8(const In* p, float (&v)[8]) {
-  if constexpr (sizeof(In) == 4) {
-    const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
-    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-  } else {
-    unpack8<In>(*reinterpret_cast<const uint4*>(p), v);
-  }
-}
-
 // 64 x 64 tile of the input per block of 256 threads; E is a 16-bit type, In any floating type.
 template <typename In, typename E>
 __global__ void __launch_bounds__(256)
@@ -275,6 +282,36 @@ normalize_vec_kernel(const In* x, const float* norm, E* out, E* out_t, int rows,
     if (trow < pcol && tcol < prow)
       *reinterpret_cast<uint4*>(secondary + (size_t(b) * pcol + trow) * prow + tcol) =
           *reinterpret_cast<const uint4*>(tile_t + c * 128 + ((uint32_t(p) * 16u) ^ swz16(c)));
+  }
+}
+
+// A = E(x * inv) in x's own orientation, zero padded from (rows x cols) to (m x n); n is a multiple of 8.  One
+// 16-byte store per thread and step; loads are vectors when x's rows are (template flag), else single elements.
+// HBM bound: one read of x, one write of A.
+template <typename In, typename E, bool VEC>
+__global__ void __launch_bounds__(256)
+normalize_rows_kernel(const In* x, const float* norm, E* out, int rows, int cols, int m, int n, float eps) {
+  pdl_wait();
+  const int b = blockIdx.y;
+  const float nb = norm ? norm[b] : 1.f;
+  const float inv = nb == 0.f ? 0.f : 1.f / fmaxf(nb, eps);
+  const In* src = x + size_t(b) * rows * cols;
+  uint4* dst = reinterpret_cast<uint4*>(out + size_t(b) * m * n);
+  const unsigned per_row = unsigned(n) / 8u;
+  const size_t total = size_t(m) * per_row;
+  for (size_t i = size_t(blockIdx.x) * 256 + threadIdx.x; i < total; i += size_t(gridDim.x) * 256) {
+    const int row = int(i / per_row), col = int(i - size_t(row) * per_row) * 8;
+    float v[8];
+    if (VEC && row < rows && col + 8 <= cols) {
+      load8<In>(src + size_t(row) * cols + col, v);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = (row < rows && col + j < cols) ? widen<In>(src[size_t(row) * cols + col + j]) : 0.f;
+    }
+    alignas(16) E e[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) e[j] = round_to<E>(__fmul_rn(v[j], inv));
+    dst[i] = *reinterpret_cast<const uint4*>(e);
   }
 }
 

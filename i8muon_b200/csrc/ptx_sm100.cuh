@@ -222,10 +222,12 @@ enum MmaKind : int { KIND_F16 = 0, KIND_TF32 = 1, KIND_I8 = 2, KIND_F8 = 3 };
 // 128 bytes wide and stored with the 128-byte swizzle that the TMA writes:
 // 8-row groups are 1024 bytes apart (stride byte offset), the leading byte
 // offset is unused for swizzled K-major tiles, descriptor version 1.
-__device__ __forceinline__ uint64_t make_smem_desc_sw128(uint32_t saddr) {
+// For an MN-major tile (rows of 128 bytes along M / N, eight k rows per 1024-byte atom) the leading byte offset is
+// the distance to the next 128 bytes along M / N.
+__device__ __forceinline__ uint64_t make_smem_desc_sw128(uint32_t saddr, uint32_t leading_bytes = 16) {
   uint64_t d = 0;
   d |= static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4);
-  d |= static_cast<uint64_t>(1) << 16;             // leading byte offset (ignored)
+  d |= static_cast<uint64_t>((leading_bytes & 0x3FFFFu) >> 4) << 16;   // ignored for K-major tiles
   d |= static_cast<uint64_t>(1024 >> 4) << 32;     // stride byte offset
   d |= static_cast<uint64_t>(1) << 46;             // version
   d |= static_cast<uint64_t>(2) << 61;             // SWIZZLE_128B
