@@ -103,17 +103,16 @@ __device__ __forceinline__ float2 unpack2<__nv_bfloat16>(uint32_t v) {
 template <typename E, int MODE>
 struct EpiFloat {
   static constexpr bool IS_F32 = sizeof(E) == 4;
+  static constexpr int STORE = MODE;
   static constexpr int E_CODE = std::is_same<E, __half>::value ? DT_F16 : (IS_F32 ? DT_F32 : DT_BF16);
   static constexpr int KIND = IS_F32 ? KIND_TF32 : KIND_F16;
   using Elem = E;
   static constexpr int PARTS = IS_F32 ? 2 : 1;
   static constexpr bool BLOCKQ = false;
-  // FP32: fold the TMEM accumulator into registers after every K block (32 elements of
-  // K, 12 tensor-core accumulations).  The tensor core accumulates with truncation:
-  // measured bias of a whole-K Gram diagonal is about -1e-8 * K relative, which at
-  // K = 4096 alone would exceed the 1e-5 bar of this path.
+  // FP32: the TMEM accumulator is folded into registers after every K block (32 elements of K, 12 tensor-core
+  // accumulations; fp32_cluster_kernel).  The tensor core accumulates with truncation: measured bias of a whole-K Gram
+  // diagonal is about -1e-8 * K relative, which at K = 4096 alone would exceed the 1e-5 bar of this path.
   static constexpr int PROMOTE_KB = IS_F32 ? 1 : 0;
-  static constexpr int NBUF = IS_F32 ? 2 : 1;
   static constexpr int EPI_WARPS = 4;
   static constexpr int STAGES = 3;
   static constexpr int MIN_CTAS = IS_F32 ? 1 : 2;
@@ -269,7 +268,7 @@ struct EpiFloat {
   template <class Acc>
   static __device__ __forceinline__ void run(const GemmGeom& g, const Args& a, const TileCtx& t,
                                              const Acc& acc) {
-    if constexpr (!IS_F32 && !Acc::IN_REGS) {
+    if constexpr (!IS_F32) {
       if (fast_ok(g, a, t)) {   // uniform over the tile's warps
         if (t.row0 + TILE > g.lm || t.col0 + TILE > g.ln) run_fast<true>(g, a, t, acc);
         else run_fast<false>(g, a, t, acc);
@@ -403,13 +402,8 @@ struct EpiFloat {
         }
       }
     };
-    if constexpr (Acc::IN_REGS) {
-#pragma unroll
-      for (int c = 0; c < TILE / 32; ++c) body(c);
-    } else {
 #pragma unroll 1
-      for (int c = t.c_begin; c < t.c_end; ++c) body(c);
-    }
+    for (int c = t.c_begin; c < t.c_end; ++c) body(c);
     if constexpr (MODE == MODE_FINAL) {
       if (a.amax != nullptr) {
         __syncwarp();

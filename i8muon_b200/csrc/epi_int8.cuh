@@ -41,7 +41,6 @@ struct EpiI8 {
   static constexpr int PARTS = 1;
   static constexpr bool BLOCKQ = false;
   static constexpr int PROMOTE_KB = 0;
-  static constexpr int NBUF = 1;
   static constexpr int EPI_WARPS = 4;
   static constexpr int STAGES = 3;
   static constexpr int MIN_CTAS = 2;
@@ -193,12 +192,10 @@ struct EpiI8 {
   template <class Acc>
   static __device__ __forceinline__ void run(const GemmGeom& g, const Args& a, const TileCtx& t,
                                              const Acc& acc) {
-    if constexpr (!Acc::IN_REGS) {
-      if (fast_ok(g, a, t)) {   // uniform over the tile's warps
-        if (t.row0 + TILE > g.lm || t.col0 + TILE > g.ln) run_fast<true>(g, a, t, acc);
-        else run_fast<false>(g, a, t, acc);
-        return;
-      }
+    if (fast_ok(g, a, t)) {   // uniform over the tile's warps
+      if (t.row0 + TILE > g.lm || t.col0 + TILE > g.ln) run_fast<true>(g, a, t, acc);
+      else run_fast<false>(g, a, t, acc);
+      return;
     }
     const bool row_ok = t.row < g.m;
     int imax = 0;

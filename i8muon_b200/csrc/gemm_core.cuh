@@ -13,13 +13,9 @@
 //   warp 1      allocates tensor memory and issues tcgen05.mma (one elected thread)
 //   warps 2..5  epilogue: tcgen05.ld the accumulator rows and run the fused epilogue
 //
-// Two accumulator disciplines:
-//   * whole-K accumulation (floating point and global-scale INT8): one 128-column
-//     accumulator, epilogue runs once after the last K block;
-//   * per-K-block promotion (128x128 block-quantised INT8 / E4M3): every 128-deep
-//     K block lands in a fresh accumulator (two TMEM buffers, ping-pong) and the
-//     epilogue warps fold it into FP32 registers with the block scales while the
-//     tensor core works on the next block.
+// The whole K extent accumulates in one 128-column accumulator (16-bit floating point and global-scale INT8) and the
+// epilogue runs once after the last K block.  Products that promote every K block into FP32 registers have kernels of
+// their own: bq_split_kernel / bq_persistent_kernel (block-quantised) and fp32_cluster_kernel (two-plane FP32).
 //
 // A debug core (geom.debug_simt) replaces TMA/tcgen05 by plain global-memory dot
 // products inside the epilogue threads, so that epilogue logic can be validated
@@ -226,7 +222,6 @@ __device__ inline uint32_t simt_dot(const GemmGeom& g, int b, int row, int col, 
 // Whole-K accumulator: chunk c = columns [32c, 32c+32) of this thread's row.
 template <int KIND, typename Elem, bool DEBUG>
 struct AccWholeK {
-  static constexpr bool IN_REGS = false;
   const GemmGeom& g;
   const TileCtx& t;
   uint32_t taddr;  // TMEM address of (lane quarter base, column 0)
@@ -243,25 +238,12 @@ struct AccWholeK {
   }
 };
 
-// Accumulator already folded into registers (chunked promotion): same chunk
-// interface, compile-time indexing so that the array stays in registers.
-struct AccRegs {
-  static constexpr bool IN_REGS = true;
-  const float (&total)[TILE];
-  __device__ __forceinline__ void load(int c, uint32_t (&v)[32]) const {
-#pragma unroll
-    for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(total[c * 32 + j]);
-  }
-};
-
 // ------------------------------------------------------------------ kernel
 // Epi supplies:
 //   KIND, Elem, PARTS (operand planes per side: 1, or 2 for split-TF32),
-//   PROMOTE_KB (0: the whole K extent accumulates in tensor memory; n > 0: every n
-//   K blocks the partial accumulator is folded into FP32 registers by the epilogue
-//   warps while the tensor core fills the other TMEM buffer), BLOCKQ (block-quantised
-//   epilogue: only its debug core runs here), STAGES, MIN_CTAS, IDESC, struct Args,
-//   static __device__ void run(g, args, t, acc)   (whole-K and chunked promotion)
+//   PROMOTE_KB (0: the whole K extent accumulates in tensor memory; otherwise only the
+//   debug core runs here), BLOCKQ (block-quantised epilogue), STAGES, MIN_CTAS, IDESC, struct Args,
+//   static __device__ void run(g, args, t, acc)
 //   static __device__ void run_debug(g, args, t)  (BLOCKQ)
 // DEBUG = true is the test-only core: no TMA / tcgen05, the epilogue threads compute
 // plain dot products.  It is a separate instantiation so that the product kernels
@@ -282,13 +264,8 @@ ns_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                const __grid_constant__ CUtensorMap map_a2, const __grid_constant__ CUtensorMap map_b2,
                GemmGeom g, typename Epi::Args args) {
   constexpr int STAGES = Epi::STAGES;
-  constexpr int PARTS = Epi::PARTS;
-  constexpr int STAGE_BYTES = 2 * PARTS * TILE_BYTES;
-  constexpr int PROMOTE = Epi::PROMOTE_KB;
-  constexpr int NBUF = Epi::NBUF;          // TMEM accumulators of 128 columns
-  constexpr int TMEM_COLS = 128 * NBUF;
-  static_assert(NBUF == 1 || NBUF == 2 || NBUF == 4, "TMEM allocations are powers of two");
-  constexpr int BKE = 128 / int(sizeof(typename Epi::Elem));  // elements per 128-byte K block
+  constexpr int STAGE_BYTES = 2 * Epi::PARTS * TILE_BYTES;
+  constexpr int TMEM_COLS = TILE;          // one accumulator of 128 columns
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -327,7 +304,8 @@ ns_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   const uint32_t smem_base = smem_u32(smem);
   constexpr int EPI_WARP0 = WarpLayout<Epi>::EPI_WARP0;
 
-  static_assert(!Epi::BLOCKQ || DEBUG, "block-quantised GEMMs run in bq_persistent_kernel");
+  static_assert(DEBUG || (!Epi::BLOCKQ && Epi::PARTS == 1),
+                "block-quantised products run in bq_split_kernel, two-plane FP32 products in fp32_cluster_kernel");
   if (warp < EPI_WARP0) {
   if (!DEBUG && warp == 0 && lane == 0) {
     // ------------------------------------------------------------ producer
@@ -345,11 +323,7 @@ ns_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       const uint32_t dst = smem_base + uint32_t(s * STAGE_BYTES);
       mbar_arrive_expect_tx(bar, STAGE_BYTES);
       Tiles::load_a(dst, &map_a, bar, kb, row0, b);
-      Tiles::load_b(dst + PARTS * TILE_BYTES, &map_b, bar, kb, col0, b);
-      if constexpr (PARTS == 2) {
-        tma_load_3d(dst + TILE_BYTES, &map_a2, bar, kb * BKE, row0, b);
-        tma_load_3d(dst + 3 * TILE_BYTES, &map_b2, bar, kb * BKE, col0, b);
-      }
+      Tiles::load_b(dst + TILE_BYTES, &map_b, bar, kb, col0, b);
       issued = kb + 1;
     }
     });
@@ -373,55 +347,21 @@ ns_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       const int s = kb % STAGES;
       ok = mbar_wait(smem_u32(&ctrl->full[s]), uint32_t(kb / STAGES) & 1u, abort_flag);
       if (!ok) break;
-      uint32_t d = tmem_base;
-      bool chunk_first = kb == 0;
-      [[maybe_unused]] bool chunk_last = false;
-      [[maybe_unused]] int buf = 0;
-      if constexpr (PROMOTE > 0) {
-        const int chunk = kb / PROMOTE;
-        buf = chunk % NBUF;
-        const int use = chunk / NBUF;  // how often this buffer has been filled before
-        chunk_first = (kb % PROMOTE) == 0;
-        chunk_last = (kb % PROMOTE) == PROMOTE - 1 || kb == g.num_kb - 1;
-        if (chunk_first) {
-          // a buffer is free until its first reuse
-          if (use >= 1)
-            ok = mbar_wait(smem_u32(&ctrl->acc_empty[buf]), uint32_t(use - 1) & 1u, abort_flag);
-          if (!ok) break;
-        }
-        d = tmem_base + uint32_t(buf * TILE);
-      }
       tc_fence_after();
       const uint32_t sa = smem_base + uint32_t(s * STAGE_BYTES);
-      const uint32_t sb = sa + PARTS * TILE_BYTES;
+      const uint32_t sb = sa + TILE_BYTES;
       const uint64_t adesc = Tiles::desc_a(sa);
       const uint64_t bdesc = Tiles::desc_b(sb);
 #pragma unroll
       for (int ks = 0; ks < 4; ++ks) {
-        uint32_t accumulate = (chunk_first && ks == 0) ? 0u : 1u;
-        umma<Epi::KIND>(d, adesc + uint64_t(ks) * Tiles::A_STEP, bdesc + uint64_t(ks) * Tiles::B_STEP,
+        uint32_t accumulate = (kb == 0 && ks == 0) ? 0u : 1u;
+        umma<Epi::KIND>(tmem_base, adesc + uint64_t(ks) * Tiles::A_STEP, bdesc + uint64_t(ks) * Tiles::B_STEP,
                         Epi::IDESC | Tiles::IDESC_BITS, accumulate);
-        if constexpr (PARTS == 2) {
-          const uint64_t adv = uint64_t(ks * 2);   // both planes K-major
-          // split-TF32: hi*hi (above) + hi*lo + lo*hi
-          const uint64_t a2 = make_smem_desc_sw128(sa + TILE_BYTES) + adv;
-          const uint64_t b2 = make_smem_desc_sw128(sb + TILE_BYTES) + adv;
-          umma<Epi::KIND>(d, adesc + adv, b2, Epi::IDESC, 1u);
-          umma<Epi::KIND>(d, a2, bdesc + adv, Epi::IDESC, 1u);
-#ifdef I8M_TF32_LOLO
-          umma<Epi::KIND>(d, a2, b2, Epi::IDESC, 1u);
-#endif
-        }
       }
       umma_commit(smem_u32(&ctrl->empty[s]));
-      if constexpr (PROMOTE > 0) {
-        if (chunk_last) umma_commit(smem_u32(&ctrl->acc_full[buf]));
-      }
     }
     });
-    if constexpr (PROMOTE == 0) {
-      if (ok) umma_commit(smem_u32(&ctrl->acc_full[0]));
-    }
+    if (ok) umma_commit(smem_u32(&ctrl->acc_full[0]));
     if (!ok) atomicCAS(g.status, 0u, unsigned(ST_MMA_TIMEOUT) | unsigned(blockIdx.x & 0xff));
   }
   } else {
@@ -438,45 +378,6 @@ ns_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     const uint32_t taddr = tmem_base + (uint32_t(t.q * 32) << 16);
     if constexpr (Epi::BLOCKQ) {
       Epi::run_debug(g, args, t);
-    } else if constexpr (PROMOTE > 0) {
-      if constexpr (DEBUG) {
-        AccWholeK<Epi::KIND, typename Epi::Elem, true> acc{g, t, taddr};
-        Epi::run(g, args, t, acc);
-      } else {
-        // Chunked promotion: the tensor core accumulates with truncation, so a
-        // long K extent is folded into registers (round-to-nearest adds) every
-        // PROMOTE K blocks.
-        float total[TILE];
-#pragma unroll
-        for (int j = 0; j < TILE; ++j) total[j] = 0.f;
-        const int chunks = (g.num_kb + PROMOTE - 1) / PROMOTE;
-        bool ok = true;
-#pragma unroll 1
-        for (int c = 0; c < chunks; ++c) {
-          const int buf = c % NBUF;
-          ok = mbar_wait(smem_u32(&ctrl->acc_full[buf]), uint32_t(c / NBUF) & 1u, abort_flag);
-          ok = __all_sync(0xffffffffu, ok);
-          if (!ok) break;
-          tc_fence_after();
-#pragma unroll
-          for (int cc = 0; cc < TILE / 32; ++cc) {
-            uint32_t v[32];
-            tmem_ld32(taddr + uint32_t(buf * TILE + cc * 32), v);
-            tmem_wait_ld();
-#pragma unroll
-            for (int j = 0; j < 32; ++j) total[cc * 32 + j] = __fadd_rn(total[cc * 32 + j], __uint_as_float(v[j]));
-          }
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(smem_u32(&ctrl->acc_empty[buf]));
-        }
-        if (ok) {
-          AccRegs acc{total};
-          Epi::run(g, args, t, acc);
-        } else if (lane == 0) {
-          atomicCAS(g.status, 0u, unsigned(ST_EPILOGUE_TIMEOUT) | unsigned(blockIdx.x & 0xff));
-        }
-      }
     } else {
       bool ok = true;
       if constexpr (!DEBUG) {

@@ -8,6 +8,7 @@
 #include <atomic>
 #include <cstdarg>
 #include <cstdio>
+#include <utility>
 
 namespace i8m {
 
@@ -45,14 +46,21 @@ int fail(int code, const char* fmt, ...);   // records the message of i8m_last_e
 // predecessor in the stream still runs and waits on the device (pdl_wait) before it touches global memory, so
 // launch latency and the prologue lie under the predecessor's tail.  The caller's LAUNCH_CHECK reads the error.
 template <typename... P, typename... A>
-inline void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
-  cudaLaunchAttribute attribute;
-  attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attribute.val.programmaticStreamSerializationAllowed = 1;
+inline void launch_clusters(void (*kernel)(P...), unsigned cluster, dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                            A&&... args) {
+  cudaLaunchAttribute attributes[2];
+  attributes[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attributes[0].val.programmaticStreamSerializationAllowed = 1;
+  attributes[1].id = cudaLaunchAttributeClusterDimension;
+  attributes[1].val.clusterDim.x = cluster; attributes[1].val.clusterDim.y = 1; attributes[1].val.clusterDim.z = 1;
   cudaLaunchConfig_t config{};
   config.gridDim = grid; config.blockDim = block; config.dynamicSmemBytes = smem; config.stream = stream;
-  config.attrs = &attribute; config.numAttrs = 1;
+  config.attrs = attributes; config.numAttrs = cluster > 1 ? 2 : 1;
   cudaLaunchKernelEx(&config, kernel, P(args)...);
+}
+template <typename... P, typename... A>
+inline void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+  launch_clusters(kernel, 1, grid, block, smem, stream, std::forward<A>(args)...);
 }
 // Dynamic shared memory above 48 KB is allowed once per kernel and device, not once per launch.
 struct SmemAllowed { std::atomic<unsigned long long> devices{0}; };

@@ -1,9 +1,12 @@
 // Launch templates of the GEMM kernels: one place that fills the geometry, encodes the operand maps and picks the
 // kernel for an epilogue.
 #pragma once
+#include <climits>
+
 #include "host.cuh"
 #include "gemm_bq_persistent.cuh"
 #include "gemm_bq_split.cuh"
+#include "gemm_fp32_cluster.cuh"
 #include "gemm_wholek_persistent.cuh"
 #include "gemm_wholek_wide.cuh"
 
@@ -26,6 +29,65 @@ inline bool narrow_units(long long tiles, long long pairs, int k_blocks, int cta
   return one < two;
 }
 
+// How many clusters of an FP32 kernel are resident at one time (asked once per device); 0 if none fits.
+template <class K>
+int resident_clusters(std::atomic<int> (&cache)[64], K* kernel, int cluster) {
+  int device = 0, n = 0;
+  if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) device = 0;
+  if ((n = cache[device].load(std::memory_order_relaxed)) > 0) return n;
+  cudaLaunchAttribute attribute;
+  attribute.id = cudaLaunchAttributeClusterDimension;
+  attribute.val.clusterDim.x = unsigned(cluster); attribute.val.clusterDim.y = 1; attribute.val.clusterDim.z = 1;
+  cudaLaunchConfig_t config{};
+  config.gridDim = dim3(unsigned(cluster)); config.blockDim = dim3(F32C_THREADS); config.dynamicSmemBytes = F32C_SMEM;
+  config.attrs = &attribute; config.numAttrs = 1;
+  if (cudaOccupancyMaxActiveClusters(&n, kernel, &config) != cudaSuccess || n < 1) {
+    cudaGetLastError();
+    return 0;
+  }
+  cache[device].store(n, std::memory_order_relaxed);
+  return n;
+}
+
+// FP32: a product of `tiles` output tiles, the K blocks of a tile split over SPLIT CTAs of a cluster.
+struct F32Call { const CUtensorMap *a, *b, *a2, *b2; const GemmGeom* g; const FloatArgs* args; long long tiles; cudaStream_t stream; };
+// The estimate of a split in nanoseconds: waves of clusters, each the K blocks of one CTA (0.75 us, measured) and the end
+// of a tile (about 5 us: prologue, sum, stores).  Measured for 1, 2, 4, 8 CTAs a tile, in us: 10 tiles x 64 K blocks 53.5,
+// 30.3, 18.5, 13.9; 36 x 128 (Gram of 1024 x 4096) 100, 54, 59, 55; 144 x 128 107, 112, 147, 184; 156 x 192 339, 245,
+// 222, 273: with few tiles a split fills the GPU, with a nearly empty last wave it evens the waves out, otherwise it
+// only adds ends of tiles.  Clusters of 4 and 8 leave some SMs out (GPC sizes), which the number of resident ones knows.
+template <int MODE, int SPLIT>
+int f32_cost(const F32Call& c, long long& cost) {
+  auto kernel = fp32_cluster_kernel<MODE, SPLIT>;
+  static SmemAllowed allowed;
+  static std::atomic<int> resident[64];
+  if (int rc = allow_smem(allowed, kernel, F32C_SMEM)) return rc;
+  const int n = resident_clusters(resident, kernel, SPLIT);
+  if (n < 1 || SPLIT > c.g->num_kb || c.tiles * SPLIT > 0x7fffffffLL) { cost = SPLIT == 1 ? LLONG_MAX - 1 : LLONG_MAX; return 0; }
+  cost = (c.tiles + n - 1) / n * (((c.g->num_kb + SPLIT - 1) / SPLIT) * 750LL + 5000);
+  return 0;
+}
+template <int MODE, int SPLIT>
+int launch_f32_split(const F32Call& c, const char* name) {
+  launch_clusters(fp32_cluster_kernel<MODE, SPLIT>, SPLIT, dim3(unsigned(c.tiles * SPLIT)), F32C_THREADS, F32C_SMEM, c.stream,
+                  *c.a, *c.b, *c.a2, *c.b2, *c.g, *c.args);
+  LAUNCH_CHECK(name);
+  return 0;
+}
+template <int MODE>
+int launch_f32(const F32Call& c, const char* name) {
+  long long cost[4];
+  if (int rc = f32_cost<MODE, 1>(c, cost[0])) return rc;
+  if (int rc = f32_cost<MODE, 2>(c, cost[1])) return rc;
+  if (int rc = f32_cost<MODE, 4>(c, cost[2])) return rc;
+  if (int rc = f32_cost<MODE, 8>(c, cost[3])) return rc;
+  int best = int(std::min_element(cost, cost + 4) - cost);
+  if (best == 3) return launch_f32_split<MODE, 8>(c, name);
+  if (best == 2) return launch_f32_split<MODE, 4>(c, name);
+  if (best == 1) return launch_f32_split<MODE, 2>(c, name);
+  return launch_f32_split<MODE, 1>(c, name);
+}
+
 // One product: operands, extents and what the kernels need besides the epilogue's own arguments.
 struct GemmCall {
   const void *a = nullptr, *a_lo = nullptr, *b = nullptr, *b_lo = nullptr;   // low planes: FP32 as two TF32 planes
@@ -42,6 +104,7 @@ int launch_gemm(const GemmCall& c, const typename Epi::Args& args, const char* n
   if (batch < 1 || m < 1 || n < 1 || k < 1) return fail(I8M_E_ARGUMENT, "%s: empty problem", name);
   if (!c.a || !c.b || !c.status) return fail(I8M_E_ARGUMENT, "%s: null operand or status pointer", name);
   if (sym && m != n) return fail(I8M_E_ARGUMENT, "%s: symmetric product needs m == n", name);
+  if (c.a_mn && !c.b_mn) return fail(I8M_E_ARGUMENT, "%s: no kernel reads only the left operand across K", name);
   constexpr int ES = int(sizeof(typename Epi::Elem));
   constexpr int STAGE_BYTES = 2 * Epi::PARTS * TILE_BYTES;
   constexpr size_t SMEM = size_t(Epi::STAGES) * STAGE_BYTES + sizeof(Ctrl) + 1024;
@@ -93,8 +156,11 @@ int launch_gemm(const GemmCall& c, const typename Epi::Args& args, const char* n
       return 0;
     }
   }
+  if constexpr (Epi::PARTS == 2) {
+    if (!g_debug_simt) return launch_f32<Epi::STORE>(F32Call{&ma, &mb, &ma2, &mb2, &g, &args, blocks, stream}, name);
+  }
   auto kernel = ns_gemm_kernel<Epi, true>;
-  if constexpr (!Epi::BLOCKQ) {
+  if constexpr (!Epi::BLOCKQ && Epi::PARTS == 1) {
     if (!g_debug_simt) kernel = ns_gemm_kernel<Epi, false>;
   }
   static SmemAllowed allowed[2];

@@ -295,7 +295,8 @@ __device__ __forceinline__ void setmaxnreg_dec() {
 // are visible; a kernel calls it in every thread before its first access to global memory, after what needs
 // none (barrier initialisation, TMEM allocation, descriptor prefetch).  There is no early trigger
 // (griddepcontrol.launch_dependents) on purpose: with it at the top of every kernel the waiting blocks slowed
-// the running grid by 3-5 % (FP32 1024 x 4096 call 1715 -> 1843 us, INT8 16 x 4096^2 17.45 -> 18.04 ms).
+// the running grid by 3-5 % (FP32 1024 x 4096 call 1715 -> 1843 us, INT8 16 x 4096^2 17.45 -> 18.04 ms), and with it where
+// a GEMM has issued its last copy and where a pass begins, a step over 768-wide matrices took 1449 instead of 1320 us.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Named barrier among a subset of warps (id 1..15; id 0 is __syncthreads).
