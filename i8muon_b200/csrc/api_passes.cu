@@ -160,30 +160,55 @@ extern "C" int i8m_normalize(const void* x, int in_dtype, const float* norm, voi
   return 0;
 }
 
+namespace {
+// One CTA-sized piece of an elementwise pass: grid-stride, about eight waves at most.
+unsigned flat_blocks(long long quads) { return unsigned(std::min<long long>(cdiv(quads, 1024), 8LL * 148)); }
+
+// a8 or a8_t may be null: only the other one is written then
+int input_quant_any(const void* x, int in_dtype, const float* amax, const float* norm, int8_t* a8, int8_t* a8_t, float* a_scale,
+                    int batch, int rows, int cols, int lp, int hp, int transpose, float eps, cudaStream_t stream) {
+  const int prow = transpose ? hp : lp, pcol = transpose ? lp : hp;
+  int8_t* same = transpose ? a8_t : a8;
+  int8_t* other = transpose ? a8 : a8_t;
+  const bool aligned = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(a8) | reinterpret_cast<uintptr_t>(a8_t)) & 15u) == 0;
+  const bool unpadded = rows == prow && cols == pcol && aligned;
+  const float e = norm ? eps : 0.f;
+  if (unpadded && other == nullptr) {
+    const long long quads = (long long)rows * cols / 4;
+    DISPATCH_IN(in_dtype, In, (launch(input_quant_flat_kernel<In>, dim3(flat_blocks(quads), batch), 256, 0, stream,
+                                  static_cast<const In*>(x), amax, norm, reinterpret_cast<uint32_t*>(same), a_scale, quads, e)));
+  } else if (unpadded && rows % 128 == 0 && cols % 128 == 0) {
+    // whole 128 x 128 tiles: vector loads, packed stores, transposes in registers
+    DISPATCH_IN(in_dtype, In, (launch(input_quant128_kernel<In>, dim3(cols / 128, rows / 128, batch), 256, 0, stream,
+                                  static_cast<const In*>(x), amax, norm, same, other, a_scale, rows, cols, e)));
+  } else {
+    dim3 grid(cdiv(pcol, 32), cdiv(prow, 32), batch);
+    DISPATCH_IN(in_dtype, In, (launch(input_quant_kernel<In>, grid, 256, 0, stream, static_cast<const In*>(x), amax, norm,
+                                  a8, a8_t, a_scale, rows, cols, lp, hp, transpose, e)));
+  }
+  LAUNCH_CHECK("input_quant");
+  return 0;
+}
+}  // namespace
+int i8m::input_quant(const void* x, int in_dtype, const float* amax, const float* norm, int8_t* a8, float* a_scale, int batch,
+                     int rows, int cols, int lp, int hp, int transpose, float eps, cudaStream_t stream) {
+  return input_quant_any(x, in_dtype, amax, norm, a8, nullptr, a_scale, batch, rows, cols, lp, hp, transpose, eps, stream);
+}
+int i8m::output_quant(const float* input, const float* maximum, int8_t* out, float* scale, int batch, int m, int n,
+                      cudaStream_t stream) {
+  const long long quads = (long long)m * n / 4;   // m and n are padded to multiples of 16
+  launch(input_quant_flat_kernel<float>, dim3(flat_blocks(quads), batch), 256, 0, stream, input, maximum,
+         static_cast<const float*>(nullptr), reinterpret_cast<uint32_t*>(out), scale, quads, -1.f);
+  LAUNCH_CHECK("output_quant");
+  return 0;
+}
 extern "C" int i8m_input_quant(const void* x, int in_dtype, const float* amax, const float* norm,
                                int8_t* a8, int8_t* a8_t, float* a_scale, int batch, int rows,
                                int cols, int lp, int hp, int transpose, float eps,
                                i8m_stream_t stream) {
   if (!x || !amax || !a8 || !a8_t || !a_scale || !float_dtype_ok(in_dtype) || batch < 1 || batch > 65535)
     return fail(I8M_E_ARGUMENT, "input_quant: bad argument");
-  const int prow = transpose ? hp : lp, pcol = transpose ? lp : hp;
-  if (rows == prow && cols == pcol && rows % 128 == 0 && cols % 128 == 0 &&
-      ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(a8) | reinterpret_cast<uintptr_t>(a8_t)) & 15u) == 0) {
-    // unpadded input of whole 128 x 128 tiles: vector loads, packed stores, transposes in registers
-    int8_t* same = transpose ? a8_t : a8;
-    int8_t* other = transpose ? a8 : a8_t;
-    DISPATCH_IN(in_dtype, In, (launch(input_quant128_kernel<In>, dim3(cols / 128, rows / 128, batch), 256, 0, S(stream),
-                                  static_cast<const In*>(x), amax, norm, same, other, a_scale, rows, cols,
-                                  norm ? eps : 0.f)));
-    LAUNCH_CHECK("input_quant");
-    return 0;
-  }
-  dim3 grid(cdiv(pcol, 32), cdiv(prow, 32), batch);
-  DISPATCH_IN(in_dtype, In, (launch(input_quant_kernel<In>, grid, 256, 0, S(stream),
-                                static_cast<const In*>(x), amax, norm, a8, a8_t, a_scale, rows, cols,
-                                lp, hp, transpose, norm ? eps : 0.f)));
-  LAUNCH_CHECK("input_quant");
-  return 0;
+  return input_quant_any(x, in_dtype, amax, norm, a8, a8_t, a_scale, batch, rows, cols, lp, hp, transpose, eps, S(stream));
 }
 
 extern "C" int i8m_symmetric_quant(const void* input, const void* maximum, const float* orig_scale,

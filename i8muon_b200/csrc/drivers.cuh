@@ -20,6 +20,15 @@ int float_gemm(const FloatGemm& g);
 int float_gemm_to_bq(const void* left, const void* right, int right_mn, void* q, void* q_t, float* scale, int compute,
                      int user_dtype, int batch, int m, int n, int k, int lm, int ln, int lp, int hp, unsigned* status,
                      cudaStream_t stream);
+// i8m_i8_gemm whose right operand may be stored with its rows along K, (batch, k, n) (b_mn set)
+int i8_gemm(int mode, const signed char* a, const signed char* b, int b_mn, const signed char* row_b, void* out, void* maximum,
+            const float* a_scale, const float* b_scale, const float* diag, int batch, int m, int n, int k, int lm, int ln,
+            float alpha, float beta, int final, int transpose, int out_dtype, unsigned* status, cudaStream_t stream);
+// i8m_input_quant and i8m_output_quant without the transposed copy
+int input_quant(const void* x, int in_dtype, const float* amax, const float* norm, signed char* a8, float* a_scale, int batch,
+                int rows, int cols, int lp, int hp, int transpose, float eps, cudaStream_t stream);
+int output_quant(const float* input, const float* maximum, signed char* out, float* scale, int batch, int m, int n,
+                 cudaStream_t stream);
 // final fold of per-chunk partials (i8m_stats layout) into norm[b] and amax[b]; either may be null
 int fold_stats(const float* partials, int batch, long long count, float* norm, float* amax, cudaStream_t stream);
 // r[b][i][i] += shift for i < logical, r (batch, m, m) in a 16-bit compute type

@@ -387,7 +387,6 @@ int run_int8(const NsCall& c, Bump& ws, bool plan, const void* x, int steps, con
   const int transpose = rows > cols;
   const size_t wide = size_t(B) * lp * hp, sq = size_t(B) * lp * lp;
   int8_t* a8 = ws.take_n<int8_t>(wide);
-  int8_t* a8t = ws.take_n<int8_t>(wide);
   float* work = ws.take_n<float>(wide);      // int32 Gram / fp32 polynomial / fp32 update
   int8_t* s8 = ws.take_n<int8_t>(sq);         // quantised Gram, then quantised polynomial
   float* a_scale = ws.take_n<float>(B);
@@ -409,8 +408,8 @@ int run_int8(const NsCall& c, Bump& ws, bool plan, const void* x, int steps, con
     if (int rc = call_stats(c, x, B, (long long)rows * cols, scratch, sbytes, normalize_input ? norm : nullptr, amax))
       return rc;
   }
-  if (int rc = i8m_input_quant(x, c.dtype, given_amax ? given_amax : amax, normalize_input ? norm : nullptr, a8, a8t, a_scale, B,
-                               rows, cols, lp, hp, transpose, c.eps, c.stream))
+  if (int rc = input_quant(x, c.dtype, given_amax ? given_amax : amax, normalize_input ? norm : nullptr, a8, a_scale, B, rows,
+                           cols, lp, hp, transpose, c.eps, c.stream))
     return rc;
   for (int it = 0; it < steps; ++it) {
     // A completed-square row (c, p, q) is the same five stages with the Gram diagonal shifted
@@ -440,12 +439,13 @@ int run_int8(const NsCall& c, Bump& ws, bool plan, const void* x, int steps, con
       return rc;
     const bool final = it == steps - 1;
     pick(2);
-    if (int rc = i8m_i8_gemm(factored ? 4 : 2, s8, a8t, a8, final ? c.out : static_cast<void*>(work), ymax, p_scale,
+    // X is stored once: the update reads it across K
+    if (int rc = i8_gemm(factored ? 4 : 2, s8, a8, 1, a8, final ? c.out : static_cast<void*>(work), ymax, p_scale,
                              a_scale, p_diag, B, lp, hp, lp, l, h, gain, 0, final, transpose, c.dtype,
                              c.status, c.stream))
       return rc;
     if (!final)
-      if (int rc = i8m_output_quant(work, ymax, a8, a8t, a_scale, B, lp, hp, c.stream)) return rc;
+      if (int rc = output_quant(work, ymax, a8, a_scale, B, lp, hp, c.stream)) return rc;
   }
   return 0;
 }
@@ -461,7 +461,6 @@ int run_int8_cubic(const NsCall& c, Bump& ws, bool plan) {
   const int cubics = c.steps - 2;
   const size_t wide = size_t(B) * lp * hp, sq = size_t(B) * lp * lp;
   int8_t* a8 = ws.take_n<int8_t>(wide);
-  int8_t* a8t = ws.take_n<int8_t>(wide);
   float* work = ws.take_n<float>(wide);
   int8_t* s8 = ws.take_n<int8_t>(sq);
   float* a_scale = ws.take_n<float>(B);
@@ -484,7 +483,7 @@ int run_int8_cubic(const NsCall& c, Bump& ws, bool plan) {
   CUDA_TRY(cudaMemsetAsync(maxima, 0, slots * B * sizeof(float), c.stream));
   if (int rc = call_stats(c, c.x, B, (long long)rows * cols, scratch, sbytes, norm, amax)) return rc;
   if (int rc = clamp_divide(norm, B, c.eps, input_gain, c.stream)) return rc;
-  if (int rc = i8m_input_quant(c.x, c.dtype, amax, norm, a8, a8t, a_scale, B, rows, cols, lp, hp, transpose, 0.f, c.stream))
+  if (int rc = input_quant(c.x, c.dtype, amax, norm, a8, a_scale, B, rows, cols, lp, hp, transpose, 0.f, c.stream))
     return rc;
   for (int i = 0; i < cubics; ++i) {
     const float gain = float(c.coeffs[3 * (i + 1)]), shift = float(c.coeffs[3 * (i + 1) + 1]);
@@ -495,10 +494,10 @@ int run_int8_cubic(const NsCall& c, Bump& ws, bool plan) {
       return rc;
     if (int rc = i8m_symmetric_quant(work, gmax, a_scale, nullptr, s8, g_scale, g_diag, B, lp, 0, shift, 0, 0, c.stream))
       return rc;
-    if (int rc = i8m_i8_gemm(4, s8, a8t, a8, work, ymax, g_scale, a_scale, g_diag, B, lp, hp, lp, l, h, -gain, 0, 0, 0, 0,
+    if (int rc = i8_gemm(4, s8, a8, 1, a8, work, ymax, g_scale, a_scale, g_diag, B, lp, hp, lp, l, h, -gain, 0, 0, 0, 0,
                              c.status, c.stream))
       return rc;
-    if (int rc = i8m_output_quant(work, ymax, a8, a8t, a_scale, B, lp, hp, c.stream)) return rc;
+    if (int rc = output_quant(work, ymax, a8, a_scale, B, lp, hp, c.stream)) return rc;
   }
   const double* abc = c.coeffs + 3 * (c.steps - 1);
   float* gmax = maxima + size_t(2 * cubics) * B;
@@ -513,7 +512,7 @@ int run_int8_cubic(const NsCall& c, Bump& ws, bool plan) {
   if (int rc = i8m_symmetric_quant(work, pmax, g_scale, g_diag, s8, p_scale, p_diag, B, lp, 1, float(abc[0]), float(abc[1]),
                                    float(abc[2]), c.stream))
     return rc;
-  return i8m_i8_gemm(2, s8, a8t, a8, c.out, nullptr, p_scale, a_scale, p_diag, B, lp, hp, lp, l, h, 0, 0, 1, transpose,
+  return i8_gemm(2, s8, a8, 1, a8, c.out, nullptr, p_scale, a_scale, p_diag, B, lp, hp, lp, l, h, 0, 0, 1, transpose,
                      c.dtype, c.status, c.stream);
 }
 

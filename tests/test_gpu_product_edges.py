@@ -3,7 +3,7 @@ import pytest
 import torch
 
 import gpu_helpers as H
-from i8muon_b200 import CutlassNSInt8, check_status, recommend_coefficients
+from i8muon_b200 import CutlassNSInt8, check_status, native, recommend_coefficients
 from oracle import ns_oracle as o
 
 pytestmark = pytest.mark.gpu
@@ -93,3 +93,21 @@ def test_16bit_calls_in_both_orientations(cuda_device, precision, batch, l, h):
             ref = o.ns_float(v, C5, 1e-7, precision, norm=norm.cpu().numpy()).double()
             assert y.shape == v.shape and y.dtype == dtype
             assert bool(((y.double().cpu() - ref).norm(dim=(1, 2)) < 2e-2 * ref.norm(dim=(1, 2))).all())
+
+
+# whole and clipped tiles, one, odd and even tile columns, extents that are no multiple of 16, the flat and the tiled quantiser
+@pytest.mark.parametrize("shape", [(1, 16, 16), (2, 128, 384), (2, 127, 129), (3, 255, 400), (1, 400, 255), (1, 1030, 130), (2, 512, 256)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_int8_updates_that_read_x_across_k(cuda_device, shape, dtype):
+    """Integer products are exact, so a whole call is the same bit for bit with plain dot products (the debug core) in the
+    place of the tensor core's reading of X with its rows along K."""
+    x = (torch.randn(shape, generator=torch.Generator().manual_seed(sum(shape))) * 0.02).to(dtype).to(cuda_device)
+    engine = CutlassNSInt8(fp16_first=False)
+    got = engine._regular_i8(x, C5, 1e-7, True, "int8")
+    native.call("i8m_set_debug_core", 1)
+    try:
+        want = engine._regular_i8(x, C5, 1e-7, True, "int8")
+    finally:
+        native.call("i8m_set_debug_core", 0)
+    check_status()
+    assert torch.equal(got, want)
