@@ -30,8 +30,8 @@ from torch.optim.optimizer import Optimizer, ParamsT
 
 from . import native
 from .coefficients import DEFAULT_COEFFICIENTS, recommend_coefficients
-from .engine import (CutlassNSInt8, coefficient_array, gram_order, on_device, post_status, raise_if_reported, raw_stream,
-                     status_host, status_word)
+from .engine import (_STATUS_HOST, CutlassNSInt8, coefficient_array, gram_order, on_device, post_status,
+                     raise_if_reported, raw_stream, status_host, status_word)
 from .routing import (EPS, GRAM_ASPECT_THRESHOLD, adjust_lr, matrix_spec, normalize_precision,
                       validate_ns_device)
 
@@ -351,6 +351,8 @@ def muon_step(
         takes_stats = isinstance(ns_engine, CutlassNSInt8) and deterministic and len(shape) == 2
         per_tensor = shape.numel()
         leading = per_tensor // (M * N)
+        # an entry point that was replaced on the engine object is called as before
+        own_entry = getattr(ns_fn, "__func__", ns_fn) is getattr(CutlassNSInt8, getattr(ns_fn, "__name__", ""), None)
         chunk = max(1, min(len(members), MAX_GROUP_BYTES // max(1, per_tensor * grads[members[0]].element_size()),
                            65535 // max(1, leading)))
         with on_device(device.index):
@@ -367,7 +369,7 @@ def muon_step(
                         c = p.contiguous(); copy_back.append((p, c)); p = c
                     g_list.append(g); b_list.append(b); p_list.append(p)
                 count = len(part)
-                if whole_groups:
+                if whole_groups and own_entry:
                     plan, block_bytes = _group_plan(ns_engine, ns_fn.__name__, actual, settings, array, device, gdtype,
                                                     pdtype, shape, count, leading, takes_stats)
                     if callable(adjust_lr_fn):
@@ -439,14 +441,18 @@ def _group_plan(engine, name, precision, settings, array, device, gdtype, pdtype
         route, compute, alignment, checked, fp16_first = engine.call_spec(name, precision)
         matrix_spec((count, *shape), gdtype, device, checked, alignment)
         _, steps, eps, deterministic, mu, mu2, nesterov, decay_mode, _, variants = settings
+        # pinned memory is not allocated under a capture: a plan first made there posts no status word and is not kept
+        posts = device.index in _STATUS_HOST or not torch.cuda.is_current_stream_capturing()
         plan = native.GroupPlan(
             count=count, leading=leading, rows=shape[-2], cols=shape[-1], grad_dtype=native.torch_dtype_code(gdtype),
             param_dtype=native.torch_dtype_code(pdtype), route=route, compute=compute, steps=steps,
             fp16_first=int(bool(fp16_first)), deterministic=int(bool(deterministic)), variants=variants,
             nesterov=int(nesterov), use_stats=int(takes_stats), decay_mode=decay_mode, eps=float(eps),
             buf_weight=1.0 - mu2, mu=mu, coeffs=array, gram_order=order.encode() if order else None,
-            status_device=status_word(device).data_ptr(), status_host=status_host(device.index).data_ptr())
+            status_device=status_word(device).data_ptr(), status_host=status_host(device.index).data_ptr() if posts else None)
         hit = ctypes.byref(plan), native.group_bytes(plan), plan, array   # the array lives as long as the plan
+        if not posts:
+            return hit[0], hit[1]
         if len(engine._group_plans) >= MAX_GROUP_PLANS:
             engine._group_plans.clear()
         engine._group_plans[key] = hit
