@@ -51,7 +51,8 @@ def test_an_entry_point_replaced_on_the_engine_is_called(cuda_device):
         muon = Muon(params, lr=0.02, weight_decay=0.01, precision="float16")
         if replaced:
             muon._ns._regular_prec = types.MethodType(entry, muon._ns)
+            muon._ns._routes.clear()          # routes looked up before the replacement keep what they found
         muon.step()
         results.append([p.detach() for p in params])
-    assert calls == [(2, 64, 96)]
+    assert len(calls) == 1 and calls[0][-2:] == (64, 96)
     assert all(torch.equal(a, b) for a, b in zip(*results))
