@@ -292,4 +292,22 @@ class CutlassNSInt8:
         return self._call("_regular_bq", x, coeffs, eps, deterministic, precision, out, stats)
 
 
+# What stands between a routed entry point and the library, as this file defines it.
+_OWN_CODE = {name: CutlassNSInt8.__dict__[name] for name in (
+    "_regular_prec", "_gram_prec", "_regular_i8", "_regular_bq", "_call", "_run", "call_spec")}
+
+
+def runs_own_code(engine) -> bool:
+    """Whether every entry point of ``engine`` does what this file says: no subclass, and nothing replaced on the
+    class or on the object.  Only then may a caller go to the library without calling them."""
+    return (type(engine) is CutlassNSInt8 and _OWN_CODE.keys().isdisjoint(engine.__dict__)
+            and all(CutlassNSInt8.__dict__.get(name) is code for name, code in _OWN_CODE.items()))
+
+
+def is_own_entry(engine, function) -> bool:
+    """Whether ``function``, as the router returned it, is this engine's own entry point of that name."""
+    code = _OWN_CODE.get(getattr(function, "__name__", None))
+    return code is not None and getattr(function, "__self__", None) is engine and getattr(function, "__func__", None) is code
+
+
 __all__ = ["CutlassNSInt8", "check_status", "status_word", "status_host", "post_status", "raise_if_reported"]

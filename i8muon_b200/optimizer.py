@@ -30,8 +30,8 @@ from torch.optim.optimizer import Optimizer, ParamsT
 
 from . import native
 from .coefficients import DEFAULT_COEFFICIENTS, recommend_coefficients
-from .engine import (_STATUS_HOST, CutlassNSInt8, coefficient_array, gram_order, on_device, post_status,
-                     raise_if_reported, raw_stream, status_host, status_word)
+from .engine import (_STATUS_HOST, CutlassNSInt8, coefficient_array, gram_order, is_own_entry, on_device, post_status,
+                     raise_if_reported, raw_stream, runs_own_code, status_host, status_word)
 from .routing import (EPS, GRAM_ASPECT_THRESHOLD, adjust_lr, matrix_spec, normalize_precision,
                       validate_ns_device)
 
@@ -330,9 +330,9 @@ def muon_step(
     decay_mode = 0 if weight_decay == 0 else (2 if weight_decay_mode == "adjusted_lr" else 1)
     decay = {0: 0.0, 2: weight_decay}.get(decay_mode, 1.0 - weight_decay if weight_decay_mode == "absolute"
                                           else 1.0 - lr * weight_decay)
-    # this library's own engine with its default kernel selection: a group is one native call
-    own_engine = type(ns_engine) is CutlassNSInt8
-    whole_groups = own_engine and not use_cuda_graph and not ns_engine.autotune and not ns_engine.tiles
+    # this library's own engine with its default kernel selection: a group is one native call.  Code that a caller has
+    # put in the place of the engine's own is called instead.
+    whole_groups = runs_own_code(ns_engine) and not use_cuda_graph and not ns_engine.autotune and not ns_engine.tiles
     if whole_groups:
         array, steps = coefficient_array(DEFAULT_COEFFICIENTS if ns_coefficients is None else ns_coefficients)
         settings = (ctypes.addressof(array), steps, eps, deterministic, mu, mu2, nesterov, decay_mode,
@@ -351,8 +351,7 @@ def muon_step(
         takes_stats = isinstance(ns_engine, CutlassNSInt8) and deterministic and len(shape) == 2
         per_tensor = shape.numel()
         leading = per_tensor // (M * N)
-        # an entry point that was replaced on the engine object is called as before
-        own_entry = getattr(ns_fn, "__func__", ns_fn) is getattr(CutlassNSInt8, getattr(ns_fn, "__name__", ""), None)
+        native_group = whole_groups and is_own_entry(ns_engine, ns_fn)
         chunk = max(1, min(len(members), MAX_GROUP_BYTES // max(1, per_tensor * grads[members[0]].element_size()),
                            65535 // max(1, leading)))
         with on_device(device.index):
@@ -369,7 +368,7 @@ def muon_step(
                         c = p.contiguous(); copy_back.append((p, c)); p = c
                     g_list.append(g); b_list.append(b); p_list.append(p)
                 count = len(part)
-                if whole_groups and own_entry:
+                if native_group:
                     plan, block_bytes = _group_plan(ns_engine, ns_fn.__name__, actual, settings, array, device, gdtype,
                                                     pdtype, shape, count, leading, takes_stats)
                     if callable(adjust_lr_fn):

@@ -1,4 +1,6 @@
 """The native plans of the optimizer's shape groups: what is kept, and when the engine's own entry points are bypassed."""
+import contextlib
+import functools
 import types
 
 import pytest
@@ -8,6 +10,62 @@ from i8muon_b200 import CutlassNSInt8, Muon, optimizer, recommend_coefficients
 from i8muon_b200.engine import coefficient_array
 
 C5 = recommend_coefficients(5)
+
+
+@pytest.fixture
+def host_only(monkeypatch):
+    """``muon_step`` on CPU tensors with the library's calls recorded instead of made: the host's decisions alone."""
+    calls = []
+    word = torch.zeros(1, dtype=torch.int32)
+
+    def call(name, *args):
+        calls.append((name, args))
+    monkeypatch.setattr(optimizer.native, "call", call)
+    monkeypatch.setattr(optimizer.native, "group_bytes", lambda plan: calls.append(("group_bytes", ())) or 256)
+    monkeypatch.setattr(optimizer, "validate_ns_device", lambda *a: None)
+    monkeypatch.setattr(optimizer, "matrix_spec", lambda *a: None)
+    monkeypatch.setattr(optimizer, "on_device", lambda index: contextlib.nullcontext())
+    monkeypatch.setattr(optimizer, "raw_stream", lambda index: 0)
+    monkeypatch.setattr(optimizer, "status_word", lambda device: word)
+    monkeypatch.setattr(optimizer, "status_host", lambda index: word)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    return calls
+
+
+def step(engine, shapes=((64, 96),) * 2, **settings):
+    tensors = [[torch.ones(s) for s in shapes] for _ in range(3)]
+    optimizer.muon_step(*tensors, **{**dict(lr=0.02, weight_decay=0.01, momentum=(0.95, 0.95), ns_coefficients=C5, eps=1e-7,
+                                            adjust_lr_fn="none", precision="float16", ns_engine=engine), **settings})
+
+
+# where a caller can put code of their own between the optimizer and the library
+@pytest.mark.parametrize("where,name,precision", [
+    ("class", "_regular_prec", "float16"), ("class", "_regular_bq", "fp8"), ("class", "_run", "float16"),
+    ("class", "_call", "int8"), ("instance", "_regular_i8", "int8"), ("instance", "_run", "float16"),
+    ("instance", "_call", "float16"), ("router", "_regular_prec", "float16")])
+def test_code_put_in_place_of_the_engines_own_is_called(monkeypatch, host_only, where, name, precision):
+    engine, seen = CutlassNSInt8(), []
+    if where == "router":                     # routes to the entry point of another engine
+        other = CutlassNSInt8(fp16_first=False)
+        monkeypatch.setattr(other, "_run", lambda route, x, *args: seen.append(x.shape) or x.clone())
+        engine.router = other.router
+    else:
+        own = getattr(CutlassNSInt8, name)
+
+        @functools.wraps(own)                 # keeps the name
+        def wrapper(*args, **kwargs):
+            x = next(a for a in args if isinstance(a, torch.Tensor))
+            seen.append(x.shape)
+            return x.clone()
+        monkeypatch.setattr(CutlassNSInt8 if where == "class" else engine, name, wrapper)
+    step(engine, precision=precision)
+    assert [tuple(s)[-2:] for s in seen] == [(64, 96)]
+    assert "i8m_group_step" not in [c[0] for c in host_only]
+
+
+def test_an_engine_as_it_comes_takes_one_native_call_per_group(host_only):
+    step(CutlassNSInt8(), ((64, 96), (64, 96), (32, 32)))
+    assert [c[0] for c in host_only if c[0] != "group_bytes"] == ["i8m_group_step"] * 2
 
 
 @pytest.mark.parametrize("known", [False, True])
