@@ -289,6 +289,8 @@ class CutlassNSInt8:
                     stats=None):
         """128x128 block-quantised NS: INT8 honours fp16_first, E4M3 never does
         (src/i8muon/_cutlass.py:71-76)."""
+        if normalize_precision(precision) in ("int8_bq", "int8"):
+            return self._regular_i8(x, coeffs, eps, deterministic, "int8", block=True, out=out, stats=stats)
         return self._call("_regular_bq", x, coeffs, eps, deterministic, precision, out, stats)
 
 

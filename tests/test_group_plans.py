@@ -41,7 +41,8 @@ def step(engine, shapes=((64, 96),) * 2, **settings):
 # where a caller can put code of their own between the optimizer and the library
 @pytest.mark.parametrize("where,name,precision", [
     ("class", "_regular_prec", "float16"), ("class", "_regular_bq", "fp8"), ("class", "_run", "float16"),
-    ("class", "_call", "int8"), ("instance", "_regular_i8", "int8"), ("instance", "_run", "float16"),
+    ("class", "_call", "int8"), ("class", "_regular_i8", "int8_bq"), ("instance", "_regular_i8", "int8"),
+    ("instance", "_regular_i8", "int8_bq"), ("instance", "_run", "float16"),
     ("instance", "_call", "float16"), ("router", "_regular_prec", "float16")])
 def test_code_put_in_place_of_the_engines_own_is_called(monkeypatch, host_only, where, name, precision):
     engine, seen = CutlassNSInt8(), []
