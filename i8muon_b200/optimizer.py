@@ -337,7 +337,7 @@ def muon_step(
         array, steps = coefficient_array(DEFAULT_COEFFICIENTS if ns_coefficients is None else ns_coefficients)
         settings = (ctypes.addressof(array), steps, eps, deterministic, mu, mu2, nesterov, decay_mode,
                     ns_engine.fp16_first, ns_engine.kernel_variants)
-    posted = set()           # devices whose status word the groups' own update kernels have posted
+    unposted = set()         # devices on which kernels were queued after the last copy of the status word to the host
 
     for (device, gdtype, pdtype, shape), members in groups.items():
         M, N = shape[-2], shape[-1]
@@ -378,7 +378,7 @@ def muon_step(
                     native.call("i8m_group_step", plan, pointers(*[g.data_ptr() for g in g_list]),
                                 pointers(*[b.data_ptr() for b in b_list]), pointers(*[p.data_ptr() for p in p_list]),
                                 block.data_ptr(), block_bytes, decay, -_as_float(adjusted), raw_stream(device.index))
-                    posted.add(device)
+                    unposted.discard(device)
                     for original, contiguous in copy_back:
                         original.copy_(contiguous)
                     continue
@@ -420,11 +420,11 @@ def muon_step(
                             ortho.data_ptr(), per_tensor, native.torch_dtype_code(pdtype),
                             native.torch_dtype_code(gdtype), decay_mode, decay, -_as_float(adjusted),
                             raw_stream(device.index))
+                unposted.add(device)
                 for original, contiguous in copy_back:
                     original.copy_(contiguous)
-    for device in {key[0] for key in groups}:
-        if device.type == "cuda" and device not in posted:
-            post_status(device)
+    for device in unposted:
+        post_status(device)
 
 
 _P_ARRAYS: dict = {}      # count -> ctypes array type

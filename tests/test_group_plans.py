@@ -28,6 +28,7 @@ def host_only(monkeypatch):
     monkeypatch.setattr(optimizer, "raw_stream", lambda index: 0)
     monkeypatch.setattr(optimizer, "status_word", lambda device: word)
     monkeypatch.setattr(optimizer, "status_host", lambda index: word)
+    monkeypatch.setattr(optimizer, "post_status", lambda device: None)
     monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
     return calls
 
@@ -67,6 +68,23 @@ def test_code_put_in_place_of_the_engines_own_is_called(monkeypatch, host_only, 
 def test_an_engine_as_it_comes_takes_one_native_call_per_group(host_only):
     step(CutlassNSInt8(), ((64, 96), (64, 96), (32, 32)))
     assert [c[0] for c in host_only if c[0] != "group_bytes"] == ["i8m_group_step"] * 2
+
+
+@pytest.mark.parametrize("shapes,posts", [(((64, 96), (32, 32)), 1), (((32, 32), (64, 96)), 0), (((64, 96), (64, 96)), 0),
+                                          (((32, 32), (32, 32)), 1)])
+def test_the_last_kernels_of_a_step_are_followed_by_a_copy_of_the_status_word(monkeypatch, host_only, shapes, posts):
+    """A native group posts the word with its own last kernel; what runs after it on the device needs another copy."""
+    posted = []
+    monkeypatch.setattr(optimizer, "post_status", posted.append)
+    engine = CutlassNSInt8()
+
+    def router(rows, cols, precision, use_gram, threshold):
+        if rows == 32:
+            return (lambda x, **kwargs: x.clone()), "float16"
+        return engine._regular_prec, "float16"
+    engine.router = router
+    step(engine, shapes)
+    assert len(posted) == posts
 
 
 @pytest.mark.parametrize("known", [False, True])
