@@ -156,6 +156,11 @@ class CutlassNSInt8:
         self._group_plans = {}   # native plans of the optimizer's shape groups (optimizer.py)
         self._factory = KernelFactory(autotune)
 
+    def __getstate__(self):
+        """What a copy or a pickle of the engine carries: its settings and measurements.  The tables below hold
+        addresses of this process (status words, coefficient arrays) and are built again where they are needed."""
+        return {**self.__dict__, "_routes": {}, "_specs": {}, "_group_plans": {}}
+
     # ------------------------------------------------------------ routing
     def router(self, M: int, N: int, precision: str, use_gram: bool, gram_aspect_threshold: float):
         key = (M, N, precision, use_gram, gram_aspect_threshold)

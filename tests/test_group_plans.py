@@ -1,6 +1,8 @@
 """The native plans of the optimizer's shape groups: what is kept, and when the engine's own entry points are bypassed."""
 import contextlib
+import copy
 import functools
+import pickle
 import types
 
 import pytest
@@ -85,6 +87,19 @@ def test_the_last_kernels_of_a_step_are_followed_by_a_copy_of_the_status_word(mo
     engine.router = router
     step(engine, shapes)
     assert len(posted) == posts
+
+
+@pytest.mark.parametrize("duplicate", [copy.copy, copy.deepcopy, lambda engine: pickle.loads(pickle.dumps(engine))])
+def test_a_used_engine_can_be_copied_and_pickled_without_its_native_state(host_only, duplicate):
+    """Plans and kept call geometries hold addresses of this process and of this engine's tables."""
+    engine = CutlassNSInt8(fp16_first=False)
+    step(engine)
+    engine._specs[("some call",)] = (1, 64, 96, 0, 256, 0x7f0000000000)
+    twin = duplicate(engine)
+    assert twin.fp16_first is False and twin.tiles == engine.tiles
+    assert not twin._specs and not twin._group_plans and len(engine._specs) == len(engine._group_plans) == 1
+    step(twin)
+    assert [c[0] for c in host_only].count("i8m_group_step") == 2 and len(engine._group_plans) == 1
 
 
 @pytest.mark.parametrize("known", [False, True])
