@@ -729,8 +729,8 @@ extern "C" int i8m_group_bytes(const i8m_group_plan* plan, size_t* bytes) {
 }
 
 extern "C" int i8m_group_step(const i8m_group_plan* plan, const void* const* grads, void* const* bufs,
-                              void* const* params, void* block, size_t block_bytes, float decay, float neg_lr,
-                              i8m_stream_t stream) {
+                              void* const* params, void* block, size_t block_bytes, float buf_weight, float mu,
+                              float decay, float neg_lr, i8m_stream_t stream) {
   GroupLayout l;
   if (int rc = group_layout(plan, l)) return rc;
   if (!block || (reinterpret_cast<uintptr_t>(block) & 255u) != 0)
@@ -738,8 +738,8 @@ extern "C" int i8m_group_step(const i8m_group_plan* plan, const void* const* gra
   if (block_bytes < l.total) return fail(I8M_E_WORKSPACE, "group_step: block %zu < %zu bytes", block_bytes, l.total);
   char* base = static_cast<char*>(block);
   float* stats = plan->use_stats ? reinterpret_cast<float*>(base + l.stats) : nullptr;
-  if (int rc = i8m_momentum(grads, bufs, plan->count, base + l.update, l.numel, plan->grad_dtype, plan->buf_weight,
-                            plan->mu, plan->nesterov, stats, stream))
+  if (int rc = i8m_momentum(grads, bufs, plan->count, base + l.update, l.numel, plan->grad_dtype, buf_weight, mu,
+                            plan->nesterov, stats, stream))
     return rc;
   if (int rc = i8m_ns_run(plan->route, base + l.update, base + l.ortho, plan->grad_dtype, l.batch, plan->rows, plan->cols,
                           plan->compute, plan->coeffs, plan->steps, plan->eps, plan->fp16_first, plan->deterministic,

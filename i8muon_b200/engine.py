@@ -121,19 +121,31 @@ def gram_order() -> str:
 
 
 _COEFFICIENT_ARRAYS = {}
+MAX_COEFFICIENT_ARRAYS = 256
+
+
+def keep(table: dict, limit: int, key, value) -> None:
+    """Put ``value`` into a bounded table; the entry that has been there longest makes room."""
+    while len(table) >= limit:
+        table.pop(next(iter(table)), None)
+    table[key] = value
+
+
+def coefficient_rows(coeffs):
+    """The rows as tuples of floats: what a schedule is known by."""
+    return tuple([tuple(map(float, row)) for row in coeffs])
 
 
 def coefficient_array(coeffs):
     """The rows as a C array and their number; the arrays of recent schedules are kept."""
-    key = tuple([tuple(map(float, row)) for row in coeffs])
+    key = coefficient_rows(coeffs)
     hit = _COEFFICIENT_ARRAYS.get(key)
     if hit is None:
         if not key or any(len(row) != 3 for row in key):
             raise ValueError("Expected a nonempty list of (a, b, c) coefficients")
         flat = [v for row in key for v in row]
         hit = (ctypes.c_double * len(flat))(*flat), len(key)
-        if len(_COEFFICIENT_ARRAYS) < 256:
-            _COEFFICIENT_ARRAYS[key] = hit
+        keep(_COEFFICIENT_ARRAYS, MAX_COEFFICIENT_ARRAYS, key, hit)
     return hit
 
 

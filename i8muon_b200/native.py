@@ -27,7 +27,7 @@ class GroupPlan(ctypes.Structure):
     _fields_ = [*[(name, c_int) for name in (
         "count", "leading", "rows", "cols", "grad_dtype", "param_dtype", "route", "compute", "steps", "fp16_first",
         "deterministic", "variants", "nesterov", "use_stats", "decay_mode")],
-        ("eps", c_float), ("buf_weight", c_float), ("mu", c_float), ("coeffs", POINTER(c_double)),
+        ("eps", c_float), ("coeffs", POINTER(c_double)),
         ("gram_order", c_char_p), ("status_device", c_void_p), ("status_host", c_void_p)]
 
 
@@ -74,7 +74,7 @@ _SIGNATURES = {
                           c_float, _P]),
     "i8m_group_bytes": (c_int, [POINTER(GroupPlan), POINTER(c_size_t)]),
     "i8m_group_step": (c_int, [POINTER(GroupPlan), POINTER(_P), POINTER(_P), POINTER(_P), _P, c_size_t, c_float, c_float,
-                               _P]),
+                               c_float, c_float, _P]),
     "i8m_adamw": (c_int, [POINTER(_P), POINTER(_P), POINTER(_P), POINTER(_P), POINTER(c_longlong), c_int,
                           c_int, c_int, c_float, c_float, c_float, c_float, c_float, c_float, c_float, _P]),
 }

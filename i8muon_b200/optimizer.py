@@ -30,8 +30,8 @@ from torch.optim.optimizer import Optimizer, ParamsT
 
 from . import native
 from .coefficients import DEFAULT_COEFFICIENTS, recommend_coefficients
-from .engine import (_STATUS_HOST, CutlassNSInt8, coefficient_array, gram_order, is_own_entry, on_device, post_status,
-                     raise_if_reported, raw_stream, runs_own_code, status_host, status_word)
+from .engine import (_STATUS_HOST, CutlassNSInt8, coefficient_array, coefficient_rows, gram_order, is_own_entry, keep,
+                     on_device, post_status, raise_if_reported, raw_stream, runs_own_code, status_host, status_word)
 from .routing import (EPS, GRAM_ASPECT_THRESHOLD, adjust_lr, matrix_spec, normalize_precision,
                       validate_ns_device)
 
@@ -334,9 +334,9 @@ def muon_step(
     # put in the place of the engine's own is called instead.
     whole_groups = runs_own_code(ns_engine) and not use_cuda_graph and not ns_engine.autotune and not ns_engine.tiles
     if whole_groups:
-        array, steps = coefficient_array(DEFAULT_COEFFICIENTS if ns_coefficients is None else ns_coefficients)
-        settings = (ctypes.addressof(array), steps, eps, deterministic, mu, mu2, nesterov, decay_mode,
-                    ns_engine.fp16_first, ns_engine.kernel_variants)
+        rows = coefficient_rows(DEFAULT_COEFFICIENTS if ns_coefficients is None else ns_coefficients)
+        coefficients = coefficient_array(rows)
+        settings = (rows, float(eps), deterministic, nesterov, decay_mode, ns_engine.fp16_first, ns_engine.kernel_variants)
     unposted = set()         # devices on which kernels were queued after the last copy of the status word to the host
 
     for (device, gdtype, pdtype, shape), members in groups.items():
@@ -369,7 +369,7 @@ def muon_step(
                     g_list.append(g); b_list.append(b); p_list.append(p)
                 count = len(part)
                 if native_group:
-                    plan, block_bytes = _group_plan(ns_engine, ns_fn.__name__, actual, settings, array, device, gdtype,
+                    plan, block_bytes = _group_plan(ns_engine, ns_fn.__name__, actual, settings, coefficients, device, gdtype,
                                                     pdtype, shape, count, leading, takes_stats)
                     if callable(adjust_lr_fn):
                         adjusted = adjust_lr(lr, adjust_lr_fn, shape)
@@ -377,7 +377,8 @@ def muon_step(
                     block = torch.empty(block_bytes, dtype=torch.uint8, device=device)
                     native.call("i8m_group_step", plan, pointers(*[g.data_ptr() for g in g_list]),
                                 pointers(*[b.data_ptr() for b in b_list]), pointers(*[p.data_ptr() for p in p_list]),
-                                block.data_ptr(), block_bytes, decay, -_as_float(adjusted), raw_stream(device.index))
+                                block.data_ptr(), block_bytes, 1.0 - mu2, mu, decay, -_as_float(adjusted),
+                                raw_stream(device.index))
                     unposted.discard(device)
                     for original, contiguous in copy_back:
                         original.copy_(contiguous)
@@ -431,7 +432,7 @@ _P_ARRAYS: dict = {}      # count -> ctypes array type
 MAX_GROUP_PLANS = 512
 
 
-def _group_plan(engine, name, precision, settings, array, device, gdtype, pdtype, shape, count, leading, takes_stats):
+def _group_plan(engine, name, precision, settings, coefficients, device, gdtype, pdtype, shape, count, leading, takes_stats):
     """The native plan of one shape group and the bytes of scratch memory it needs (kept per engine)."""
     order = gram_order() if name == "_gram_prec" else None
     key = (name, precision, settings, device, gdtype, pdtype, shape, count, takes_stats, order)
@@ -439,22 +440,21 @@ def _group_plan(engine, name, precision, settings, array, device, gdtype, pdtype
     if hit is None:
         route, compute, alignment, checked, fp16_first = engine.call_spec(name, precision)
         matrix_spec((count, *shape), gdtype, device, checked, alignment)
-        _, steps, eps, deterministic, mu, mu2, nesterov, decay_mode, _, variants = settings
+        array, steps = coefficients
+        _, eps, deterministic, nesterov, decay_mode, _, variants = settings
         # pinned memory is not allocated under a capture: a plan first made there posts no status word and is not kept
         posts = device.index in _STATUS_HOST or not torch.cuda.is_current_stream_capturing()
         plan = native.GroupPlan(
             count=count, leading=leading, rows=shape[-2], cols=shape[-1], grad_dtype=native.torch_dtype_code(gdtype),
             param_dtype=native.torch_dtype_code(pdtype), route=route, compute=compute, steps=steps,
             fp16_first=int(bool(fp16_first)), deterministic=int(bool(deterministic)), variants=variants,
-            nesterov=int(nesterov), use_stats=int(takes_stats), decay_mode=decay_mode, eps=float(eps),
-            buf_weight=1.0 - mu2, mu=mu, coeffs=array, gram_order=order.encode() if order else None,
+            nesterov=int(nesterov), use_stats=int(takes_stats), decay_mode=decay_mode, eps=eps,
+            coeffs=array, gram_order=order.encode() if order else None,
             status_device=status_word(device).data_ptr(), status_host=status_host(device.index).data_ptr() if posts else None)
         hit = ctypes.byref(plan), native.group_bytes(plan), plan, array   # the array lives as long as the plan
         if not posts:
             return hit[0], hit[1]
-        if len(engine._group_plans) >= MAX_GROUP_PLANS:
-            engine._group_plans.clear()
-        engine._group_plans[key] = hit
+        keep(engine._group_plans, MAX_GROUP_PLANS, key, hit)
     return hit[0], hit[1]
 
 

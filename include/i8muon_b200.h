@@ -237,13 +237,13 @@ int i8m_apply(void* const* params, int count, const void* update_device, long lo
  * momentum, Newton-Schulz and decay + update of `count` same-shaped tensors (leading x rows x cols each) in one
  * call: i8m_momentum, i8m_ns_run and i8m_apply over one block of scratch memory that holds the stacked update,
  * its orthogonalised result, the statistics partials and the Newton-Schulz workspace.  What stays the same from
- * step to step is in the plan; addresses and the learning rate are arguments. */
+ * step to step is in the plan; addresses and what schedules change (momentum, decay, learning rate) are arguments. */
 typedef struct i8m_group_plan {
   int count, leading, rows, cols;
   int grad_dtype, param_dtype;
   int route, compute, steps, fp16_first, deterministic, variants;
   int nesterov, use_stats, decay_mode;
-  float eps, buf_weight, mu;
+  float eps;
   const double* coeffs;      /* steps rows of (a, b, c), host memory */
   const char* gram_order;    /* as in i8m_ns_run */
   uint32_t* status_device;
@@ -251,7 +251,8 @@ typedef struct i8m_group_plan {
 } i8m_group_plan;
 int i8m_group_bytes(const i8m_group_plan* plan, size_t* bytes);
 int i8m_group_step(const i8m_group_plan* plan, const void* const* grads, void* const* bufs, void* const* params,
-                   void* block_device, size_t block_bytes, float decay, float neg_lr, i8m_stream_t stream);
+                   void* block_device, size_t block_bytes, float buf_weight, float mu, float decay, float neg_lr,
+                   i8m_stream_t stream);
 
 /* AdamW for the parameters Muon does not take (embeddings, heads, vectors).  No counterpart in
  * the reference: its `scalar_optimizer` slot takes any torch optimizer

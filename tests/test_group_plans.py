@@ -89,6 +89,38 @@ def test_the_last_kernels_of_a_step_are_followed_by_a_copy_of_the_status_word(mo
     assert len(posted) == posts
 
 
+def test_a_momentum_schedule_keeps_one_plan(host_only):
+    engine = CutlassNSInt8()
+    for mu, mu2 in ((0.85, 0.9), (0.9, 0.95), (0.95, 0.95)):
+        step(engine, momentum=(mu, mu2))
+        name, args = host_only[-1]
+        assert name == "i8m_group_step" and args[-5:-3] == (1.0 - mu2, mu)
+    assert len(engine._group_plans) == 1 and [c[0] for c in host_only].count("group_bytes") == 1
+    step(engine, momentum=(0.9,))             # without Nesterov: another kernel argument of the plan
+    assert len(engine._group_plans) == 2
+
+
+def test_plans_survive_more_schedules_than_their_table_holds(host_only):
+    engine = CutlassNSInt8()
+    for i in range(300):
+        coefficient_array([(2.0 + i, -1.5, 0.5)])
+    late = [(9.0, -1.5, 0.5)]
+    for _ in range(3):
+        step(engine, ns_coefficients=late)
+    assert len(engine._group_plans) == 1 and [c[0] for c in host_only].count("group_bytes") == 1
+    for i in range(optimizer.MAX_GROUP_PLANS + 5):
+        step(engine, ns_coefficients=[(2.0 + i, -1.5, 0.25)])
+    assert len(engine._group_plans) == optimizer.MAX_GROUP_PLANS
+
+
+def test_an_epsilon_held_in_a_tensor_is_read_at_every_step(host_only):
+    engine, eps = CutlassNSInt8(), torch.tensor(1e-7)
+    step(engine, eps=eps)
+    eps.fill_(1e-3)
+    step(engine, eps=eps)
+    assert sorted(plan[2].eps for plan in engine._group_plans.values()) == pytest.approx([1e-7, 1e-3])
+
+
 @pytest.mark.parametrize("duplicate", [copy.copy, copy.deepcopy, lambda engine: pickle.loads(pickle.dumps(engine))])
 def test_a_used_engine_can_be_copied_and_pickled_without_its_native_state(host_only, duplicate):
     """Plans and kept call geometries hold addresses of this process and of this engine's tables."""
@@ -117,9 +149,9 @@ def test_a_plan_made_under_a_capture_allocates_no_pinned_memory(monkeypatch, kno
     monkeypatch.setattr(optimizer.native, "group_bytes", lambda plan: 256)
     monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: True)
     array, steps = coefficient_array(C5)
-    settings = (0, steps, 1e-7, True, 0.95, 0.95, True, 1, True, 0)
+    settings = (tuple(C5), 1e-7, True, True, 1, True, 0)
     engine = CutlassNSInt8()
-    plan, size = optimizer._group_plan(engine, "_regular_prec", "float16", settings, array, torch.device("cuda", 0),
+    plan, size = optimizer._group_plan(engine, "_regular_prec", "float16", settings, (array, steps), torch.device("cuda", 0),
                                        torch.float32, torch.float32, torch.Size((64, 64)), 2, 1, True)
     assert size == 256
     assert bool(plan._obj.status_host) == known and pinned == ([0] if known else [])
