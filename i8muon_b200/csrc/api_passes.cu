@@ -176,7 +176,7 @@ int input_quant_any(const void* x, int in_dtype, const float* amax, const float*
   if (unpadded && other == nullptr) {
     const long long quads = (long long)rows * cols / 4;
     DISPATCH_IN(in_dtype, In, (launch(input_quant_flat_kernel<In>, dim3(flat_blocks(quads), batch), 256, 0, stream,
-                                  static_cast<const In*>(x), amax, norm, reinterpret_cast<uint32_t*>(same), a_scale, quads, e)));
+                                  static_cast<const In*>(x), amax, norm, reinterpret_cast<uint32_t*>(same), a_scale, quads, e, 0)));
   } else if (unpadded && rows % 128 == 0 && cols % 128 == 0) {
     // whole 128 x 128 tiles: vector loads, packed stores, transposes in registers
     DISPATCH_IN(in_dtype, In, (launch(input_quant128_kernel<In>, dim3(cols / 128, rows / 128, batch), 256, 0, stream,
@@ -198,7 +198,7 @@ int i8m::output_quant(const float* input, const float* maximum, int8_t* out, flo
                       cudaStream_t stream) {
   const long long quads = (long long)m * n / 4;   // m and n are padded to multiples of 16
   launch(input_quant_flat_kernel<float>, dim3(flat_blocks(quads), batch), 256, 0, stream, input, maximum,
-         static_cast<const float*>(nullptr), reinterpret_cast<uint32_t*>(out), scale, quads, -1.f);
+         static_cast<const float*>(nullptr), reinterpret_cast<uint32_t*>(out), scale, quads, 0.f, 1);
   LAUNCH_CHECK("output_quant");
   return 0;
 }

@@ -574,18 +574,19 @@ input_quant128_kernel(const In* x, const float* amax, const float* norm, int8_t*
 // Codes of a whole matrix in its own order, four per thread and step (one 16- or 8-byte load, one 4-byte store, both
 // contiguous over a warp), four steps in flight: for products that read the codes across K instead of a transposed copy.
 // `quads` groups of four elements per matrix.  scale[b] is that of an input (amax / (127 max(norm, eps))), or with
-// eps < 0 that of a product's result (1 / (127 / maximum)).  HBM bound: one read, one write.  Writing no transposed copy
+// `of_result` that of a product's result (1 / (127 / maximum)).  HBM bound: one read, one write.  Writing no transposed copy
 // took 16 x 4096^2 INT8 from 17.24 to 16.54 ms and a step over 768-wide matrices from 1320 to 1228 us.
 template <typename In>
 __global__ void __launch_bounds__(256)
-input_quant_flat_kernel(const In* x, const float* amax, const float* norm, uint32_t* out, float* scale, long long quads, float eps) {
+input_quant_flat_kernel(const In* x, const float* amax, const float* norm, uint32_t* out, float* scale, long long quads, float eps,
+                        int of_result) {
   pdl_wait();
   const int b = blockIdx.y;
   const float mx = amax[b];
   const float nb = norm ? norm[b] : 1.f;
   const float multiplier = mx > 0.f ? 127.f / mx : 0.f;
   if (blockIdx.x == 0 && threadIdx.x == 0)
-    scale[b] = mx > 0.f ? (eps < 0.f ? 1.f / multiplier : mx / __fmul_rn(127.f, fmaxf(nb, eps))) : 0.f;
+    scale[b] = mx > 0.f ? (of_result ? 1.f / multiplier : mx / __fmul_rn(127.f, fmaxf(nb, eps))) : 0.f;
   const In* src = x + size_t(b) * size_t(quads) * 4;
   uint32_t* dst = out + size_t(b) * size_t(quads);
   for (long long first = (long long)blockIdx.x * 1024 + threadIdx.x; first < quads; first += (long long)gridDim.x * 1024) {

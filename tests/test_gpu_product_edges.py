@@ -111,3 +111,12 @@ def test_int8_updates_that_read_x_across_k(cuda_device, shape, dtype):
         native.call("i8m_set_debug_core", 0)
     check_status()
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("shape", [(2, 256, 384), (1, 100, 300)])
+def test_int8_calls_take_any_epsilon(cuda_device, shape):
+    """The norm of these inputs is far above both values, so neither takes part in the result."""
+    x = torch.randn(shape, generator=torch.Generator().manual_seed(1)).to(cuda_device)
+    engine = CutlassNSInt8(fp16_first=False)
+    assert torch.equal(engine._regular_i8(x, C5, -1.0), engine._regular_i8(x, C5, 0.0))
+    check_status()
