@@ -1,12 +1,16 @@
 // FP32 products (three TF32 products of two-plane operands) split along K over a cluster of CTAs.
 //
-// A 128 x 128 output tile belongs to a cluster of 1, 2, 4 or 8 CTAs; CTA r of it multiplies the r-th share of the
-// K blocks and parks its FP32 partial tile in its own shared memory.  After a cluster barrier CTA r finishes the
-// r-th band of 128 / size rows: it adds the partials of all CTAs in rank order (read over distributed shared
-// memory; the order is fixed, so results repeat bit for bit) and stores the band.
+// The K blocks of a 128 x 128 output tile form SEGMENTS = 1, 2, 4 or 8 segments, each summed on its own.  The sums of two
+// consecutive segments are added, then these pairs one after the other.  How many segments there are depends on one
+// matrix's extents alone (f32_segments), so a result depends neither on the batch it was computed in nor on the device.
+// How many CTAs share a tile (SPLIT, up to one per segment) is the launcher's choice and changes no bit: a CTA takes a run
+// of segments, holds sums that wait for their partner in tensor memory, and parks what it has in shared memory.  After
+// a cluster barrier CTA r finishes the r-th band of 128 / SPLIT rows: it adds up the parked sums of all CTAs in the order
+// above (read over distributed shared memory) and stores the band.
 //
 //   warp 0       TMA producer: 64 KB stages {A hi, A lo, B hi, B lo} of one 32-element K block, three deep
-//   warp 1       tcgen05.mma issuer: twelve instructions per K block into one of four 128-column accumulators
+//   warp 1       tcgen05.mma issuer: twelve instructions per K block into one of four 128-column accumulators (three or
+//                two where the CTA holds sums of earlier segments: they take 128 columns each)
 //   warps 4..11  fold: every K block's accumulator is added into FP32 registers with round-to-nearest (the tensor
 //                core accumulates with truncation), two warps per TMEM lane quarter, 64 columns per thread
 //   all warps    sum of the partials, fused epilogue, coalesced stores of every plane and orientation
@@ -15,7 +19,11 @@
 // and the copies write 64 KB, 160 KB in all, 1280 cycles at 128 bytes per cycle; measured 0.75 us, about 1430.  One CTA
 // per tile with four fold warps took 1900 (the fold's TMEM round trips are a serial chain and two accumulators left the
 // issuer waiting for it), left three quarters of the GPU idle when a product has few tiles, and stored rows with 32
-// sectors per request.  One 1024 x 4096 call 1745 -> 721 us, six of 1537 x 700 1814 -> 858 us.
+// sectors per request.  One 1024 x 4096 call 1745 -> 720 us, six of 1537 x 700 1814 -> 867 us.
+// What the fixed order of the sums costs, against adding up whatever share each CTA had: nothing for one matrix, 1 to 3 %
+// in batches (six of 1537 x 700 858 -> 867 us, 24 of 512 x 2048 1964 -> 2010), 12 % where a segment is a single K block
+// (24 of 256 x 256 205 -> 229).  Parking a segment apart wherever its partner is in another CTA's half made the tail read
+// twice the sums (two of 512 x 2048 258 -> 285); pairs need that in one place only.
 #pragma once
 #include "epi_float.cuh"
 
@@ -24,13 +32,28 @@ namespace i8m {
 constexpr int F32C_STAGES = 3;
 constexpr int F32C_STAGE_BYTES = 4 * TILE_BYTES;
 constexpr int F32C_THREADS = 384;
-constexpr int F32C_NBUF = 4;
+constexpr int F32C_TMEM_TILES = 4;     // of 128 columns: accumulators, and sums of earlier segments
+// What a CTA does with the segments it takes.
+template <int SPLIT, int SEGMENTS>
+struct F32Share {
+  static_assert(SPLIT >= 1 && SPLIT <= SEGMENTS && SEGMENTS % SPLIT == 0 && SEGMENTS <= 8, "at most one CTA per segment");
+  static constexpr int TAKEN = SEGMENTS / SPLIT;                       // segments per CTA
+  static constexpr int HELD = TAKEN == 1 ? 0 : TAKEN == 2 ? 1 : 2;     // sums in tensor memory: half a pair, earlier pairs
+  static constexpr int NBUF = F32C_TMEM_TILES - HELD;                  // accumulators
+  // Two CTAs with two pairs each: the second one's pairs follow the first one's sum one by one, so it parks them apart.
+  static constexpr bool APART = SPLIT > 1 && TAKEN > 2;
+  static_assert(!APART || (SPLIT == 2 && TAKEN == 4), "no other CTA has pairs that wait for those before them");
+  static constexpr int PARKED = APART ? 2 : 1;                         // parked tiles in a CTA's shared memory
+  static constexpr int SUMS = APART ? 3 : SPLIT;                       // parked sums of the cluster
+};
 constexpr int F32C_FOLD_WARP0 = 4, F32C_FOLD_WARPS = 8;
-// The parked partial tile: rows of 132 floats (16-byte aligned; a warp's 32 own-row vector stores cover all banks
-// evenly).  It and the band of summed rows lie over the operand ring, which is idle by then.
+// The parked tiles: rows of 132 floats (16-byte aligned; a warp's 32 own-row vector stores cover all banks
+// evenly).  They and the band of summed rows lie over the operand ring, which is idle by then.
 constexpr int F32C_PARK_PITCH = 132;
 constexpr int F32C_PARK_BYTES = TILE * F32C_PARK_PITCH * 4;
-static_assert(F32C_PARK_BYTES + TILE * TILE * 4 <= F32C_STAGES * F32C_STAGE_BYTES, "the tail overlays the ring");
+static_assert(F32C_PARK_BYTES + TILE * TILE * 4 <= F32C_STAGES * F32C_STAGE_BYTES &&
+                  2 * F32C_PARK_BYTES + TILE / 2 * TILE * 4 <= F32C_STAGES * F32C_STAGE_BYTES,
+              "the parked sums (two tiles with two CTAs per output tile, else one) and the band overlay the ring");
 constexpr size_t F32C_SMEM = size_t(F32C_STAGES) * F32C_STAGE_BYTES + sizeof(Ctrl) + 1024;
 
 __device__ __forceinline__ void cluster_sync() {
@@ -61,7 +84,7 @@ __device__ __forceinline__ uint32_t band_quad(uint32_t band, int row, int quad) 
 // band; then along the rows the sum, the polynomial and the row-major stores; then the transposed stores, as 4 x 4
 // blocks out of the band.  Shared-memory and global accesses are 16-byte vectors without bank conflicts where the
 // matrix allows it (with one scalar read per element the tail of a tile took 10 us).
-template <int MODE, int SPLIT>
+template <int MODE, int SPLIT, int SEGMENTS>
 __device__ __forceinline__ void f32c_tail(const GemmGeom& g, const FloatArgs& a, int b, int tm, int tn, uint32_t park, uint32_t band,
                                           int rank) {
   constexpr int R = TILE / SPLIT, WARPS = F32C_THREADS / 32;
@@ -77,18 +100,28 @@ __device__ __forceinline__ void f32c_tail(const GemmGeom& g, const FloatArgs& a,
   float* out = static_cast<float*>(a.out);
   float* out_lo = static_cast<float*>(a.out_lo);
 
-  uint32_t part[SPLIT];
+  using Share = F32Share<SPLIT, SEGMENTS>;
+  constexpr int SUMS = Share::SUMS;
+  uint32_t part[SUMS];
 #pragma unroll
-  for (int s = 0; s < SPLIT; ++s) part[s] = SPLIT == 1 ? park : cluster_map(park, uint32_t(s));
-  auto total4 = [&](int r, int c) {       // the four sums (r, c .. c + 3) of the tile, partials added in rank order
+  for (int s = 0; s < SUMS; ++s) {
+    const int rank_of = Share::APART && s > 0 ? 1 : s, slot = Share::APART && s == 2 ? 1 : 0;
+    part[s] = park + uint32_t(slot * F32C_PARK_BYTES);
+    if (SPLIT > 1) part[s] = cluster_map(part[s], uint32_t(rank_of));
+  }
+  auto add4 = [](float4& a, const float4& b) {
+    a.x = __fadd_rn(a.x, b.x); a.y = __fadd_rn(a.y, b.y); a.z = __fadd_rn(a.z, b.z); a.w = __fadd_rn(a.w, b.w);
+  };
+  auto total4 = [&](int r, int c) {       // the elements (r, c .. c + 3) of the tile, segments added in their order
     const uint32_t at = uint32_t(r * F32C_PARK_PITCH + c) * 4u;
-    float4 w[SPLIT];
+    float4 w[SUMS];
 #pragma unroll
-    for (int s = 0; s < SPLIT; ++s) w[s] = SPLIT == 1 ? lds128(part[s] + at) : ldc128(part[s] + at);
+    for (int s = 0; s < SUMS; ++s) w[s] = SPLIT == 1 ? lds128(part[s] + at) : ldc128(part[s] + at);
+    constexpr int PAIR = SPLIT == SEGMENTS && SPLIT > 1 ? 2 : 1;      // one sum per segment: pairs first
 #pragma unroll
-    for (int s = 1; s < SPLIT; ++s) {
-      w[0].x = __fadd_rn(w[0].x, w[s].x); w[0].y = __fadd_rn(w[0].y, w[s].y);
-      w[0].z = __fadd_rn(w[0].z, w[s].z); w[0].w = __fadd_rn(w[0].w, w[s].w);
+    for (int s = 0; s < SUMS; s += PAIR) {
+      if constexpr (PAIR == 2) add4(w[s], w[s + 1]);
+      if (s > 0) add4(w[0], w[s]);
     }
     return w[0];
   };
@@ -238,12 +271,14 @@ __device__ __forceinline__ void f32c_tail(const GemmGeom& g, const FloatArgs& a,
   }
 }
 
-template <int MODE, int SPLIT>
+template <int MODE, int SPLIT, int SEGMENTS>
 __global__ void __launch_bounds__(F32C_THREADS, 1)
 fp32_cluster_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                     const __grid_constant__ CUtensorMap map_a2, const __grid_constant__ CUtensorMap map_b2,
                     GemmGeom g, FloatArgs args) {
+  using Share = F32Share<SPLIT, SEGMENTS>;
   constexpr int STAGES = F32C_STAGES;
+  constexpr int NBUF = Share::NBUF;
   constexpr uint32_t IDESC = EpiFloat<float, MODE>::IDESC;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -262,7 +297,7 @@ fp32_cluster_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       mbar_init(smem_u32(&ctrl->full[s]), 1);
       mbar_init(smem_u32(&ctrl->empty[s]), 1);
     }
-    for (int i = 0; i < F32C_NBUF; ++i) {
+    for (int i = 0; i < NBUF; ++i) {
       mbar_init(smem_u32(&ctrl->acc_full[i]), 1);
       mbar_init(smem_u32(&ctrl->acc_empty[i]), F32C_FOLD_WARPS);
     }
@@ -274,7 +309,7 @@ fp32_cluster_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     tma_prefetch_desc(&map_b2);
   }
   if (warp == 1) {
-    tmem_alloc(smem_u32(&ctrl->tmem_base), TILE * F32C_NBUF);
+    tmem_alloc(smem_u32(&ctrl->tmem_base), TILE * F32C_TMEM_TILES);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -317,7 +352,7 @@ fp32_cluster_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     // ------------------------------------------------------------ MMA issuer
     bool ok = true;
     for (int i = 0; i < nkb; ++i) {
-      const int s = i % STAGES, buf = i % F32C_NBUF, use = i / F32C_NBUF;
+      const int s = i % STAGES, buf = i % NBUF, use = i / NBUF;
       if (use >= 1) {
         ok = mbar_wait(smem_u32(&ctrl->acc_empty[buf]), uint32_t(use - 1) & 1u, abort_flag);
         if (!ok) break;
@@ -349,10 +384,38 @@ fp32_cluster_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 #pragma unroll
     for (int j = 0; j < 64; ++j) total[j] = 0.f;
     bool ok = true;
+    // Sums that wait in tensor memory, behind the accumulators: HALF_PAIR the first segment of a pair, EARLIER the pairs
+    // before it.
+    constexpr int HALF_PAIR = 0, EARLIER = 1;
+    auto held = [&](int slot) { return taddr + uint32_t((NBUF + slot) * TILE); };
+    auto put = [&](int slot) {
+      uint32_t v[32];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(total[32 * h + j]);
+        tmem_st32(held(slot) + uint32_t(32 * h), v);
+      }
+      tmem_wait_st();
+    };
+    auto add = [&](int slot) {       // total <- held sum + total
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        uint32_t v[32];
+        tmem_ld32(held(slot) + uint32_t(32 * h), v);
+        tmem_wait_ld();
+#pragma unroll
+        for (int j = 0; j < 32; ++j) total[32 * h + j] = __fadd_rn(__uint_as_float(v[j]), total[32 * h + j]);
+      }
+    };
+    int segment = 0;                 // of this CTA's TAKEN
+    // the first K block, counted from kb0, of the next segment
+    auto segment_end = [&] { return int((long long)g.num_kb * (rank * Share::TAKEN + segment + 1) / SEGMENTS) - kb0; };
+    int end = segment_end();
 #pragma unroll 1
     for (int i = 0; i < nkb; ++i) {
-      const int buf = i % F32C_NBUF;
-      ok = mbar_wait_warp_inline(smem_u32(&ctrl->acc_full[buf]), uint32_t(i / F32C_NBUF) & 1u, abort_flag);
+      const int buf = i % NBUF;
+      ok = mbar_wait_warp_inline(smem_u32(&ctrl->acc_full[buf]), uint32_t(i / NBUF) & 1u, abort_flag);
       if (!ok) break;
       tc_fence_after();
       uint32_t v[32], w[32];
@@ -367,11 +430,43 @@ fp32_cluster_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         total[j] = __fadd_rn(total[j], __uint_as_float(v[j]));
         total[32 + j] = __fadd_rn(total[32 + j], __uint_as_float(w[j]));
       }
+      if constexpr (Share::TAKEN > 1) {
+        if (i + 1 == end && i + 1 < nkb) {               // uniform over the CTA
+          // an even segment waits for its partner; an odd one completes a pair, which joins those before it
+          const int partners = segment % 2 == 0 ? 0 : segment == 1 ? 1 : 2;
+#pragma unroll 1
+          for (int slot = 0; slot < partners; ++slot) add(slot);
+          put(segment % 2 == 0 ? HALF_PAIR : EARLIER);
+#pragma unroll
+          for (int j = 0; j < 64; ++j) total[j] = 0.f;
+          ++segment;
+          end = segment_end();
+        }
+      }
     }
     if (!ok && lane == 0) atomicCAS(g.status, 0u, unsigned(ST_EPILOGUE_TIMEOUT) | unsigned(blockIdx.x & 0xff));
     if (ok) {
       // The last accumulator is complete: every copy of this CTA has landed and been read, the ring is free.
-      const uint32_t own = smem_base + uint32_t((q * 32 + lane) * F32C_PARK_PITCH + 64 * half) * 4u;
+      uint32_t own = smem_base + uint32_t((q * 32 + lane) * F32C_PARK_PITCH + 64 * half) * 4u;
+      const bool apart = Share::APART && rank == 1;
+      if constexpr (Share::HELD > 0) {
+#pragma unroll 1
+        for (int slot = 0; slot < (apart ? 1 : Share::HELD); ++slot) add(slot);
+      }
+      if constexpr (Share::APART) {
+        if (apart) {
+          uint32_t v[32];
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            tmem_ld32(held(EARLIER) + uint32_t(32 * h), v);
+            tmem_wait_ld();
+#pragma unroll
+            for (int j = 0; j < 32; j += 4)
+              sts128u(own + 4u * uint32_t(32 * h + j), make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]));
+          }
+          own += F32C_PARK_BYTES;
+        }
+      }
 #pragma unroll
       for (int j = 0; j < 64; j += 4)
         sts128(own + 4u * uint32_t(j), make_float4(total[j], total[j + 1], total[j + 2], total[j + 3]));
@@ -383,8 +478,8 @@ fp32_cluster_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   tc_fence_before();
   if constexpr (SPLIT == 1) __syncthreads();
   else cluster_sync();
-  if (warp == 1) tmem_dealloc(tmem_base, TILE * F32C_NBUF);
-  f32c_tail<MODE, SPLIT>(g, args, b, tm, tn, smem_base, smem_base + F32C_PARK_BYTES, rank);
+  if (warp == 1) tmem_dealloc(tmem_base, TILE * F32C_TMEM_TILES);
+  f32c_tail<MODE, SPLIT, SEGMENTS>(g, args, b, tm, tn, smem_base, smem_base + Share::PARKED * F32C_PARK_BYTES, rank);
   if constexpr (SPLIT > 1) cluster_sync();   // nobody leaves while its partial tile is still being read
 }
 

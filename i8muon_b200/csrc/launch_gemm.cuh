@@ -49,43 +49,76 @@ int resident_clusters(std::atomic<int> (&cache)[64], K* kernel, int cluster) {
   return n;
 }
 
-// FP32: a product of `tiles` output tiles, the K blocks of a tile split over SPLIT CTAs of a cluster.
-struct F32Call { const CUtensorMap *a, *b, *a2, *b2; const GemmGeom* g; const FloatArgs* args; long long tiles; cudaStream_t stream; };
-// The estimate of a split in nanoseconds: waves of clusters, each the K blocks of one CTA (0.75 us, measured) and the end
-// of a tile (about 5 us: prologue, sum, stores).  Measured for 1, 2, 4, 8 CTAs a tile, in us: 10 tiles x 64 K blocks 53.5,
-// 30.3, 18.5, 13.9; 36 x 128 (Gram of 1024 x 4096) 100, 54, 59, 55; 144 x 128 107, 112, 147, 184; 156 x 192 339, 245,
-// 222, 273: with few tiles a split fills the GPU, with a nearly empty last wave it evens the waves out, otherwise it
-// only adds ends of tiles.  Clusters of 4 and 8 leave some SMs out (GPC sizes), which the number of resident ones knows.
-template <int MODE, int SPLIT>
-int f32_cost(const F32Call& c, long long& cost) {
-  auto kernel = fp32_cluster_kernel<MODE, SPLIT>;
+// FP32 products: K segments whose sums are added in order, and the CTAs that share a tile.
+//
+// One estimate serves both choices, in nanoseconds: waves of clusters, each the K blocks of one CTA (0.75 us, measured)
+// and the end of a tile (about 5 us: prologue, sum, stores).  Measured for 1, 2, 4, 8 CTAs a tile, in us: 10 tiles x 64 K
+// blocks 53.5, 30.3, 18.5, 13.9; 36 x 128 (Gram of 1024 x 4096) 100, 54, 59, 55; 144 x 128 107, 112, 147, 184; 156 x 192
+// 339, 245, 222, 273: with few tiles a split fills the GPU, with a nearly empty last wave it evens the waves out,
+// otherwise it only adds ends of tiles.
+inline long long f32_estimate(long long tiles, int resident, int num_kb, int ctas) {
+  return (tiles + resident - 1) / resident * ((num_kb + ctas - 1) / ctas * 750LL + 5000);
+}
+// How many segments the K blocks form: the split that one matrix alone would take.  A function of its extents only - not
+// of the batch, and not of the device, whose clusters (74, 33 and 15 on the B200s measured: GPC sizes leave some SMs out)
+// are constants here - because it decides the order of the sums and with it the bits of the result.
+inline int f32_segments(long long tiles_per_matrix, int num_kb) {
+  constexpr int RESIDENT[4] = {148, 74, 33, 15};
+  int best = 1;
+  long long cost = f32_estimate(tiles_per_matrix, RESIDENT[0], num_kb, 1);
+  for (int i = 1; i < 4 && (1 << i) <= num_kb; ++i) {
+    const long long c = f32_estimate(tiles_per_matrix, RESIDENT[i], num_kb, 1 << i);
+    if (c < cost) { cost = c; best = 1 << i; }
+  }
+  return best;
+}
+struct F32Call {
+  const CUtensorMap *a, *b, *a2, *b2;
+  const GemmGeom* g;
+  const FloatArgs* args;
+  long long tiles;      // of the whole batch
+  cudaStream_t stream;
+};
+// The best of SPLIT, SPLIT / 2 ... 1 CTAs per tile: `best` and `cost` come with those of the larger splits.  A cluster that
+// the device does not offer is left out; one CTA per tile needs none.
+template <int MODE, int SPLIT, int SEGMENTS>
+int f32_best_split(const F32Call& c, int& best, long long& cost) {
+  auto kernel = fp32_cluster_kernel<MODE, SPLIT, SEGMENTS>;
   static SmemAllowed allowed;
   static std::atomic<int> resident[64];
   if (int rc = allow_smem(allowed, kernel, F32C_SMEM)) return rc;
   const int n = resident_clusters(resident, kernel, SPLIT);
-  if (n < 1 || SPLIT > c.g->num_kb || c.tiles * SPLIT > 0x7fffffffLL) { cost = SPLIT == 1 ? LLONG_MAX - 1 : LLONG_MAX; return 0; }
-  cost = (c.tiles + n - 1) / n * (((c.g->num_kb + SPLIT - 1) / SPLIT) * 750LL + 5000);
+  if (n >= 1 && c.tiles * SPLIT <= 0x7fffffffLL) {
+    const long long v = f32_estimate(c.tiles, n, c.g->num_kb, SPLIT);
+    if (v <= cost) { cost = v; best = SPLIT; }
+  }
+  if constexpr (SPLIT > 1) return f32_best_split<MODE, SPLIT / 2, SEGMENTS>(c, best, cost);
   return 0;
 }
-template <int MODE, int SPLIT>
-int launch_f32_split(const F32Call& c, const char* name) {
-  launch_clusters(fp32_cluster_kernel<MODE, SPLIT>, SPLIT, dim3(unsigned(c.tiles * SPLIT)), F32C_THREADS, F32C_SMEM, c.stream,
-                  *c.a, *c.b, *c.a2, *c.b2, *c.g, *c.args);
+template <int MODE, int SPLIT, int SEGMENTS>
+int launch_f32_split(const F32Call& c, int split, const char* name) {
+  if constexpr (SPLIT > 1)
+    if (split != SPLIT) return launch_f32_split<MODE, SPLIT / 2, SEGMENTS>(c, split, name);
+  launch_clusters(fp32_cluster_kernel<MODE, SPLIT, SEGMENTS>, SPLIT, dim3(unsigned(c.tiles * SPLIT)), F32C_THREADS, F32C_SMEM,
+                  c.stream, *c.a, *c.b, *c.a2, *c.b2, *c.g, *c.args);
   LAUNCH_CHECK(name);
   return 0;
 }
+template <int MODE, int SEGMENTS>
+int launch_f32_segments(const F32Call& c, const char* name) {
+  int split = 1;
+  long long cost = LLONG_MAX;
+  if (int rc = f32_best_split<MODE, SEGMENTS, SEGMENTS>(c, split, cost)) return rc;
+  return launch_f32_split<MODE, SEGMENTS, SEGMENTS>(c, split, name);
+}
 template <int MODE>
 int launch_f32(const F32Call& c, const char* name) {
-  long long cost[4];
-  if (int rc = f32_cost<MODE, 1>(c, cost[0])) return rc;
-  if (int rc = f32_cost<MODE, 2>(c, cost[1])) return rc;
-  if (int rc = f32_cost<MODE, 4>(c, cost[2])) return rc;
-  if (int rc = f32_cost<MODE, 8>(c, cost[3])) return rc;
-  int best = int(std::min_element(cost, cost + 4) - cost);
-  if (best == 3) return launch_f32_split<MODE, 8>(c, name);
-  if (best == 2) return launch_f32_split<MODE, 4>(c, name);
-  if (best == 1) return launch_f32_split<MODE, 2>(c, name);
-  return launch_f32_split<MODE, 1>(c, name);
+  switch (f32_segments(c.g->tiles_per_batch, c.g->num_kb)) {
+    case 8: return launch_f32_segments<MODE, 8>(c, name);
+    case 4: return launch_f32_segments<MODE, 4>(c, name);
+    case 2: return launch_f32_segments<MODE, 2>(c, name);
+    default: return launch_f32_segments<MODE, 1>(c, name);
+  }
 }
 
 // One product: operands, extents and what the kernels need besides the epilogue's own arguments.

@@ -13,6 +13,7 @@ Differences that a caller can observe:
   * ``deterministic=False`` selects one-pass statistics with atomics on every route (the reference
     only has that flavour for global INT8); the default is the two-pass reduction in a fixed order;
   * the result is a fresh tensor, not a view into the call's workspace;
+  * with ``deterministic=True`` a matrix's result has the same bits alone and in any batch, in every precision;
   * ``tiles`` selects, per product of the global-INT8 route (``aat``, ``square``, ``update``), between this
     library's kernels for whole-K products: the reference's tile id 4 (its TMA tile) maps to the
     persistent kernel with 128 x 256 units (also the default), ids 0-3 (its cp.async tiles) to the

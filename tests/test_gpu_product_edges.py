@@ -76,6 +76,34 @@ def test_fp32_products_over_all_splits(cuda_device, b, m, n, k):
     assert H.status_ok(cuda_device) == 0
 
 
+# the K blocks of these products form 8, 4, 2 and 1 segments; the batches take as many CTAs per tile, half as many and one
+@pytest.mark.parametrize("rows,cols,batches", [(100, 1500, (1, 14, 20, 40, 160)), (512, 2048, (1, 2, 4, 7, 24)), (700, 1537, (1, 2, 6)),
+                                               (1024, 1024, (1, 3)), (16, 40, (1, 300))])
+@pytest.mark.parametrize("entry", ["_regular_prec", "_gram_prec"])
+def test_fp32_results_do_not_depend_on_the_batch(cuda_device, rows, cols, batches, entry):
+    x = torch.randn(max(batches), rows, cols, generator=torch.Generator().manual_seed(rows)).to(cuda_device)
+    call = getattr(CutlassNSInt8(), entry)
+    results = [call(x[:n], C5, 1e-7, True, "float32") for n in batches]
+    check_status()
+    for y in results[1:]:
+        assert torch.equal(y[:1], results[0])
+    assert all(torch.equal(y, results[-1][:len(y)]) for y in results)
+
+
+# one matrix leaves the GPU half empty (units of one tile), the batches fill it (units of two)
+@pytest.mark.parametrize("precision", ["float16", "bfloat16", "int8", "int8_bq", "fp8"])
+@pytest.mark.parametrize("rows,cols", [(300, 700), (513, 257)])
+def test_other_results_do_not_depend_on_the_batch_either(cuda_device, rows, cols, precision):
+    x = torch.randn(40, rows, cols, generator=torch.Generator().manual_seed(rows)).to(cuda_device)
+    engine = CutlassNSInt8()
+    for gram in (False, True):
+        function, compute = engine.router(rows, cols, precision, gram, 1.0)
+        many = function(x, coeffs=C5, precision=compute)
+        for n in (1, 6):
+            assert torch.equal(function(x[:n], coeffs=C5, precision=compute), many[:n])
+    check_status()
+
+
 # extents one below, on and above a 16-bit tile; rows with no 16-byte vectors; one, odd and even tile columns
 @pytest.mark.parametrize("precision", ["float16", "bfloat16"])
 @pytest.mark.parametrize("batch,l,h", [(1, 16, 16), (2, 127, 129), (1, 128, 257), (3, 255, 385), (1, 130, 1030), (40, 192, 200)])
