@@ -44,7 +44,8 @@ def status_word(device: torch.device) -> torch.Tensor:
     index = device.index if device.index is not None else torch.cuda.current_device()
     word = _STATUS_WORDS.get(index)
     if word is None:
-        word = _STATUS_WORDS[index] = torch.zeros(1, dtype=torch.int32, device=torch.device("cuda", index))
+        # setdefault: of two threads that come here together both get the word that stays (its address is kept)
+        word = _STATUS_WORDS.setdefault(index, torch.zeros(1, dtype=torch.int32, device=torch.device("cuda", index)))
     return word
 
 
@@ -68,8 +69,7 @@ def status_host(index: int) -> torch.Tensor:
     """One int32 in pinned host memory per device, where the status word is copied to at the end of a step."""
     host = _STATUS_HOST.get(index)
     if host is None:
-        host = torch.zeros(1, dtype=torch.int32).pin_memory()
-        _STATUS_HOST[index] = host
+        host = _STATUS_HOST.setdefault(index, torch.zeros(1, dtype=torch.int32).pin_memory())
         _STATUS_VIEWS[index] = ctypes.c_int32.from_address(host.data_ptr())
     return host
 
@@ -92,7 +92,7 @@ def post_status(device) -> None:
 
 def raise_if_reported() -> None:
     """Raise if a status word copied to the host has arrived and is not zero (no synchronisation)."""
-    for index, view in _STATUS_VIEWS.items():
+    for index, view in tuple(_STATUS_VIEWS.items()):
         code = view.value
         if code != 0:
             torch.cuda.synchronize(index)   # copies still in flight land before the words are cleared

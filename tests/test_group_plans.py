@@ -3,12 +3,13 @@ import contextlib
 import copy
 import functools
 import pickle
+import threading
 import types
 
 import pytest
 import torch
 
-from i8muon_b200 import CutlassNSInt8, Muon, optimizer, recommend_coefficients
+from i8muon_b200 import CutlassNSInt8, Muon, engine as engine_module, optimizer, recommend_coefficients
 from i8muon_b200.engine import coefficient_array
 
 C5 = recommend_coefficients(5)
@@ -132,6 +133,31 @@ def test_a_used_engine_can_be_copied_and_pickled_without_its_native_state(host_o
     assert not twin._specs and not twin._group_plans and len(engine._specs) == len(engine._group_plans) == 1
     step(twin)
     assert [c[0] for c in host_only].count("i8m_group_step") == 2 and len(engine._group_plans) == 1
+
+
+@pytest.mark.parametrize("which", ["status_word", "status_host"])
+def test_threads_that_come_first_together_share_one_status_word(monkeypatch, which):
+    """Plans keep the words' addresses, so a word that one thread was given may not be replaced by another thread's."""
+    meet, real = threading.Barrier(2), torch.zeros
+
+    def zeros(*args, **kwargs):
+        meet.wait(10)                        # both threads have found no word
+        return real(*args, **{**kwargs, "device": "cpu"})
+    for table in ("_STATUS_WORDS", "_STATUS_HOST", "_STATUS_VIEWS"):
+        monkeypatch.setattr(engine_module, table, {})
+    monkeypatch.setattr(engine_module.torch, "zeros", zeros)
+    monkeypatch.setattr(torch.Tensor, "pin_memory", lambda self: self)
+    make, got = getattr(engine_module, which), []
+    argument = torch.device("cuda", 0) if which == "status_word" else 0
+    threads = [threading.Thread(target=lambda: got.append(make(argument))) for _ in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert len(got) == 2 and got[0] is got[1] is make(argument)
+    if which == "status_host":
+        got[0].fill_(7)
+        assert engine_module._STATUS_VIEWS[0].value == 7
 
 
 @pytest.mark.parametrize("known", [False, True])
