@@ -55,6 +55,16 @@ def normalize(x, norm, compute, eps=1e-7):
     return a, at, alo, atlo
 
 
+def normalize_rows(x, norm, compute, eps=1e-7):
+    """As whole 16-bit calls do it: the caller's orientation, no transposed copy."""
+    b, rows, cols = x.shape
+    m, n = -(-rows // 16) * 16, -(-cols // 16) * 16
+    a = torch.full((b, m, n), float("nan"), device=x.device, dtype=compute)
+    native.call("i8m_normalize", x.data_ptr(), DT[x.dtype], ptr(norm), a.data_ptr(), None, None, None, DT[compute], b, rows,
+                cols, m, n, 0, eps, _stream())
+    return a
+
+
 def float_gemm(left, right_t, *, mode=0, sym=False, final=False, transpose=False, out_dtype=None, lm=None,
                ln=None, coeffs=(0.0, 0.0, 0.0), want_t=False, left_lo=None, right_lo=None):
     b, m, k = left.shape

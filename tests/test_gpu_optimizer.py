@@ -362,3 +362,42 @@ def test_momentum_kernel_leaves_the_statistics_of_its_update(cuda_device, dtype,
     assert torch.equal(plain, fed)
     with pytest.raises(ValueError, match="stats must be"):
         engine._regular_bq(update, C5, 1e-7, True, "int8_bq", stats=stats[:2])
+
+
+class SeparateCalls(CutlassNSInt8):
+    """A subclass takes momentum, Newton-Schulz and update as calls of their own."""
+
+
+@pytest.mark.parametrize("precision", ["auto", "float32", "int8_bq"])
+@pytest.mark.parametrize("layout", ["plain", "strided", "folded"])
+def test_one_native_call_per_group_gives_the_bits_of_separate_calls(cuda_device, precision, layout):
+    """Non-contiguous gradients, parameters and buffers (the copies go back), leading dimensions, a side stream, and several
+    groups and chunks in one step."""
+    shapes = {"plain": [(200, 136)] * 3 + [(64, 64)], "strided": [(200, 136)] * 2 + [(96, 160)],
+              "folded": [(2, 3, 48, 80)] * 2 + [(5, 64, 32)]}[layout]
+    gen = torch.Generator().manual_seed(11)
+
+    def tensors(scale):
+        made = []
+        for shape in shapes:
+            t = (torch.randn(shape, generator=gen) * scale).to(torch.bfloat16).to(cuda_device)
+            made.append(t.mT.contiguous().mT if layout == "strided" else t)
+        return made
+    params, grads, bufs = tensors(0.02), tensors(1e-3), tensors(1e-3)
+    assert layout != "strided" or not params[0].is_contiguous()
+    results = []
+    for engine in (CutlassNSInt8(), SeparateCalls()):
+        p, g, b = [[t.clone(memory_format=torch.preserve_format) for t in ts] for ts in (params, grads, bufs)]
+        torch.cuda.synchronize()
+        stream = torch.cuda.Stream(cuda_device)
+        with torch.cuda.stream(stream):
+            for momentum in ((0.9, 0.95), (0.95,)):
+                muon_step(p, g, b, lr=0.02, weight_decay=0.01, momentum=momentum, ns_coefficients=C5, eps=1e-7,
+                          adjust_lr_fn="match_rms_adamw", ns_engine=engine, precision=precision)
+        stream.synchronize()
+        check_status()
+        results.append((p, b))
+    assert results[0][0][0].stride() == params[0].stride()
+    for ours, theirs in zip(results[0], results[1]):
+        assert all(torch.equal(x, y) for x, y in zip(ours, theirs))
+    assert not torch.equal(results[0][0][0], params[0])

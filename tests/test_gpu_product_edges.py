@@ -123,12 +123,13 @@ def test_16bit_calls_in_both_orientations(cuda_device, precision, batch, l, h):
             assert bool(((y.double().cpu() - ref).norm(dim=(1, 2)) < 2e-2 * ref.norm(dim=(1, 2))).all())
 
 
-# whole and clipped tiles, one, odd and even tile columns, extents that are no multiple of 16, the flat and the tiled quantiser
+# whole and clipped tiles, one, odd and even tile columns, extents that are no multiple of 16; wide and tall inputs
 @pytest.mark.parametrize("shape", [(1, 16, 16), (2, 128, 384), (2, 127, 129), (3, 255, 400), (1, 400, 255), (1, 1030, 130), (2, 512, 256)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_int8_updates_that_read_x_across_k(cuda_device, shape, dtype):
     """Integer products are exact, so a whole call is the same bit for bit with plain dot products (the debug core) in the
-    place of the tensor core's reading of X with its rows along K."""
+    place of the tensor core's reading of X with its rows along K.  Both calls run the same quantisers, which the stage
+    tests and the whole calls against the oracle hold."""
     x = (torch.randn(shape, generator=torch.Generator().manual_seed(sum(shape))) * 0.02).to(dtype).to(cuda_device)
     engine = CutlassNSInt8(fp16_first=False)
     got = engine._regular_i8(x, C5, 1e-7, True, "int8")

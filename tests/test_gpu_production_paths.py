@@ -1,4 +1,4 @@
-"""Bit-exact checks of the kernel paths that the benchmarked step actually runs.
+"""Bit-exact checks at sizes of the benchmarked step.
 
 The small stage tests give every persistent CTA at most one tile.  Here every launch has more tiles
 than the GPU has SMs and several K blocks per tile, so the tile loops of ``bq_persistent_kernel``
@@ -155,11 +155,26 @@ def int8_iteration_bit_exact(dev, x, coeffs):
 @pytest.mark.parametrize("shape", [(1, 2048, 2048), (1, 4096, 4096), (1, 3000, 1400)],
                          ids=["2048x2048", "4096x4096", "3000x1400-ragged-tall"])
 def test_global_int8_iteration_bit_exact_beyond_one_tile_per_cta(cuda_device, shape):
-    """2048^2: 136 Gram tiles and 256 update tiles through both streams of the whole-K persistent
-    kernel; 4096^2 is the shape of the global-INT8 benchmark configuration (528 Gram tiles, 32 K
-    blocks of 128); 3000 x 1400 has ragged edges and rows > cols."""
+    """The products and the tiled quantisers, stage by stage.  2048^2: 136 Gram tiles and 256 update tiles through both
+    streams of the whole-K persistent kernel; 4096^2 is the shape of the global-INT8 benchmark configuration (528 Gram
+    tiles, 32 K blocks of 128); 3000 x 1400 has ragged edges and rows > cols.  Whole calls quantise and read X in
+    another way: the next test."""
     x = seeded(shape, torch.float32, 73, outliers=True).to(cuda_device)
     int8_iteration_bit_exact(cuda_device, x, C6[1])
+
+
+@pytest.mark.parametrize("shape,dtype", [((1, 2304, 2304), torch.float32), ((1, 2304, 2304), torch.bfloat16),
+                                         ((2, 1400, 3000), torch.float32), ((1, 3000, 1400), torch.float32)])
+def test_whole_global_int8_calls_bit_exact(cuda_device, shape, dtype):
+    """The stage test above asks for transposed copies; a whole call stores its codes once, quantises them in a flat pass
+    and reads them across K.  Two rows (input quantiser, two updates, the quantiser between them) against the oracle
+    from the same norm.  2304^2 has more groups of four than one sweep of the flat pass (8 x 148 x 1024); the others are
+    padded.  FP32 results are the same bits, BF16 results the same values rounded once."""
+    x = seeded(shape, dtype, 77, outliers=True)
+    y = CutlassNSInt8(fp16_first=False)._regular_i8(x.to(cuda_device), C6[:2], 1e-7, True, "int8")
+    norm, _ = H.stats(x.to(cuda_device))
+    assert H.status_ok(cuda_device) == 0
+    assert torch.equal(y.cpu(), o.ns_int8(x, C6[:2], 1e-7, fp16_first=False, norm=npy(norm)))
 
 
 def test_fp16_gram_polar_express_on_the_2048x8192_shape(cuda_device, monkeypatch):

@@ -77,6 +77,23 @@ def test_normalize(cuda_device, shape, compute):
         assert torch.equal(got_t.cpu(), ref.mT)
 
 
+@pytest.mark.parametrize("shape", [(2, 48, 112), (2, 112, 48), (1, 37, 75), (3, 16, 1), (1, 201, 328), (1, 4001, 5000)])
+@pytest.mark.parametrize("compute", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+def test_normalize_into_one_copy(cuda_device, shape, compute, dtype):
+    """The pass that whole 16-bit calls use: rows of vectors and rows that start anywhere, inputs off a 16-byte boundary,
+    and more groups than one sweep of the grid."""
+    x = make_input(shape, dtype, 5).to(cuda_device)
+    norm, _ = H.stats(x)
+    b, rows, cols = shape
+    inv = torch.from_numpy(o._inv_norm(npy(norm), 1e-7)).to(cuda_device)
+    want = (x.float() * inv[:, None, None]).to(compute)          # one product and one rounding per element
+    for given in (x, shifted(x)):
+        got = H.normalize_rows(given, norm, compute)
+        assert torch.equal(got[:, :rows, :cols], want)
+        assert not got[:, rows:].any() and not got[:, :, cols:].any()
+
+
 @pytest.mark.parametrize("shape", [(2, 64, 160), (2, 160, 64), (1, 45, 91), (1, 91, 45)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_input_quant_bit_exact(cuda_device, shape, dtype):
