@@ -15,8 +15,9 @@
 //                core accumulates with truncation), two warps per TMEM lane quarter, 64 columns per thread
 //   all warps    sum of the partials, fused epilogue, coalesced stores of every plane and orientation
 //
-// What bounds it: shared memory.  A K block is 768 tensor cycles (12 x 64), but its twelve instructions read 8 KB each
-// and the copies write 64 KB, 160 KB in all, 1280 cycles at 128 bytes per cycle; measured 0.75 us, about 1430.  One CTA
+// What bounds it: a K block is 768 tensor cycles (12 x 64) and takes 0.75 us, about 1430.  Its twelve instructions read
+// 8 KB each and the copies write 64 KB, 160 KB in all, which would be 1280 cycles at 128 bytes per cycle; but the counters put
+// the shared-memory banks at a third of their peak (tensor pipe 44 % active), so the rest is not explained.  One CTA
 // per tile with four fold warps took 1900 (the fold's TMEM round trips are a serial chain and two accumulators left the
 // issuer waiting for it), left three quarters of the GPU idle when a product has few tiles, and stored rows with 32
 // sectors per request.  One 1024 x 4096 call 1745 -> 720 us, six of 1537 x 700 1814 -> 867 us.

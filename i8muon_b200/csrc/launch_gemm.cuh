@@ -21,8 +21,8 @@ inline int wide_group(long long k_bytes) {
 
 // Whether the persistent whole-K kernel takes units of one tile (128 x 128) instead of two (128 x 256).  A K block costs
 // about 540 cycles in a pair and 390 alone (both bound by what the SM takes in from L2: 48 and 32 KB at 89 bytes per
-// cycle), a tile's epilogue about 2000, of which only the last one per CTA is not under another unit's K loop.  Pairs
-// win when there are many; with few tiles the number of waves decides.
+// cycle, the measured rate of such copies), a tile's epilogue about 2000 (an estimate), of which only the last one per CTA
+// is not under another unit's K loop.  Pairs win when there are many; with few tiles the number of waves decides.
 inline bool narrow_units(long long tiles, long long pairs, int k_blocks, int ctas) {
   const long long one = (tiles + ctas - 1) / ctas * k_blocks * 390 + 2000;
   const long long two = (pairs + ctas - 1) / ctas * k_blocks * 540 + 4000;

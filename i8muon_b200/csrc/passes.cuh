@@ -234,7 +234,8 @@ normalize_kernel(const In* x, const float* norm, E* out, E* out_t, float* out_lo
 // results as the scalar kernels above.
 __device__ __forceinline__ uint32_t swz16(int c) { return uint32_t((c >> 3) & 7) << 4; }
 
-// 64 x 64 tile of the input per block of 256 threads; E is a 16-bit type, In any floating type.
+// 64 x 64 tile of the input per block of 256 threads; E is a 16-bit type, In any floating type.  For the stage entry of the
+// C ABI with a transposed copy; whole calls use normalize_rows_kernel.
 template <typename In, typename E>
 __global__ void __launch_bounds__(256)
 normalize_vec_kernel(const In* x, const float* norm, E* out, E* out_t, int rows, int cols, int m, int n,
@@ -600,7 +601,8 @@ input_quant_flat_kernel(const In* x, const float* amax, const float* norm, uint3
   }
 }
 
-// FP32 (m x n) -> int8 and transposed int8, m and n multiples of 128, 16-byte aligned pointers.
+// FP32 (m x n) -> int8 and transposed int8, m and n multiples of 128, 16-byte aligned pointers.  For the stage entry of the
+// C ABI; whole calls use input_quant_flat_kernel.
 __global__ void __launch_bounds__(256)
 output_quant128_kernel(const float* input, const float* maximum, int8_t* out, int8_t* out_t, float* scale, int m,
                        int n) {

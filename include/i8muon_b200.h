@@ -126,7 +126,8 @@ int i8m_stats_static(const void* x_device, int dtype, int batch, long long count
 
 /* ---- stage level: floating path -------------------------------------------
  * normalize: src/i8muon/csrc/prec.cu:193-208.  A = E(x / max(norm, eps)) padded to
- * (lp x hp) plus A^T; transpose != 0 means the input has rows > cols and A = x^T.
+ * (lp x hp) plus A^T (a_t NULL: A alone, as whole 16-bit calls ask for it); transpose != 0 means the input has rows > cols
+ * and A = x^T.
  * For compute_dtype F32 every matrix is a pair of planes (hi, lo) of TF32-
  * representable floats; *_lo pointers are required then and ignored otherwise. */
 int i8m_normalize(const void* x_device, int in_dtype, const float* norm_device, void* a, void* a_t,
@@ -151,7 +152,9 @@ int i8m_float_gemm_to_bq(const void* left, const void* right_t, void* q, void* q
                          int user_dtype, int batch, int m, int n, int k, int lm, int ln, int lp, int hp,
                          uint32_t* status_device, i8m_stream_t stream);
 
-/* ---- stage level: global-scale INT8 path --------------------------------- */
+/* ---- stage level: global-scale INT8 path ---------------------------------
+ * The quantisers below also write the transposed codes that b_t of i8m_i8_gemm wants.  Whole calls (i8m_ns_run) store the
+ * codes once and read them across K; the codes, scales and results are the same. */
 /* input_quant: src/i8muon/csrc/int8.cu:508-527 (norm_device NULL = no normalisation) */
 int i8m_input_quant(const void* x_device, int in_dtype, const float* amax_device,
                     const float* norm_device, int8_t* a8, int8_t* a8_t, float* a_scale, int batch,
