@@ -78,7 +78,8 @@ def test_fp32_products_over_all_splits(cuda_device, b, m, n, k):
 
 # the K blocks of these products form 8, 4, 2 and 1 segments; the batches take as many CTAs per tile, half as many and one
 @pytest.mark.parametrize("rows,cols,batches", [(100, 1500, (1, 14, 20, 40, 160)), (512, 2048, (1, 2, 4, 7, 24)), (700, 1537, (1, 2, 6)),
-                                               (1024, 1024, (1, 3)), (16, 40, (1, 300))])
+                                               (1024, 1024, (1, 3)), (16, 40, (1, 300)), (256, 256, (1, 6, 12, 40)),
+                                               (251, 256, (1, 6, 12, 40))])
 @pytest.mark.parametrize("entry", ["_regular_prec", "_gram_prec"])
 def test_fp32_results_do_not_depend_on_the_batch(cuda_device, rows, cols, batches, entry):
     x = torch.randn(max(batches), rows, cols, generator=torch.Generator().manual_seed(rows)).to(cuda_device)
